@@ -29,6 +29,7 @@
 #include "kernels.cuh"
 #include "adjoint.cuh"
 #include "direct_launch.h"
+#include "resident_launch.h"
 #include "dlayout.h"
 #include "logodds.h"
 #include "seq.cuh"
@@ -151,6 +152,13 @@ struct flbp_engine {
     int f_form = 0, v_form = 0;
     int f_grid_direct = 1, v_grid_direct = 1;
     int sms = 148;
+    // Resident run kernel: -1 not planned yet, 0 not for this graph, 1 with
+    // uncached constants, 2 with them in shared memory; its grid, rows of
+    // items per block and shared memory.
+    int res_plan = -1;
+    unsigned res_grid = 1;
+    uint32_t res_rows_f = 0, res_rows_v = 0;
+    size_t res_smem = 0;
     std::map<std::pair<int, int>, cudaGraphExec_t> graphs;  // (mode, sweeps) -> executable graph
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     float last_ms = 0.f;
@@ -743,9 +751,133 @@ void fill_info(flbp_engine *e, flbp_run_info *info, long long sweeps, long long 
     info->launches = e->launches - launches0;
 }
 
+// ---- the resident run kernel (resident.cuh)
+
+constexpr long long kResSweeps = 4096;  // sweeps per launch at most
+// Largest graphs that run resident, in device slots. Measured per FP32 sweep,
+// resident against two launches of the staged passes (three families of
+// graphs): tolerance runs 11.1 : 18.3 us at 158 k slots, 17.4 : 23.9 at
+// 635 k, 22.3 : 26.7 at 952 k but 29.3 : 27.0 with fan-ins up to 4,096 at
+// 1.0 M; fixed runs, which have no residual to reduce, 9.2 : 11.2 at 158 k,
+// 18.1 : 19.4 at 709 k, 19.6 : 18.9 at 952 k. FP64 crosses at the same sizes.
+constexpr uint64_t kResFixedSlots = 720000, kResRuleSlots = 980000;
+
+// Grid, rows and shared memory of the resident kernel for this engine's
+// graph, or a plan of 0 where the pass kernels run instead.
+template <typename T>
+void plan_resident_t(flbp_engine *e) {
+    const HostLayout &L = e->L;
+    const bool damp = e->damping != 0.0, batch = e->n_graphs > 0;
+    e->res_plan = 0;
+    if (e->n_graphs > 32u * kGroupWords) return;
+    int coop = 0;
+    if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, e->device) != cudaSuccess || !coop) return;
+    const uint32_t nfb = L.nf_big - L.nf_huge, nvb = L.nv_big - L.nv_huge;
+    const uint32_t n_f = nfb + L.n_fgroups(), n_v = nvb + L.n_vgroups();
+    const uint32_t items = std::max({n_f, n_v, 1u}), huge = std::max(L.nf_huge, L.nv_huge);
+    const uint32_t want = std::max((items + 3) / 4, std::max(huge, 1u));
+    auto rows = [&](uint32_t n, uint32_t nb) { return (n + nb - 1) / nb; };
+    for (int cache = 1; cache >= 0; cache--) {
+        // most blocks per SM first
+        for (int per = sizeof(T) == 4 ? 2 : 1; per >= 1; per--) {
+            const uint32_t nb = std::min<uint32_t>(want, (uint32_t)e->sms * (uint32_t)per);
+            const uint32_t rf = rows(n_f, nb), rv = rows(n_v, nb);
+            size_t smem = 0;
+            if (cache) {
+                if (rf + rv > kResMaxRows) continue;
+                std::vector<uint32_t> words(nb, (3u * (rf + rv) + 31u) & ~31u);
+                for (int fac = 0; fac < 2; fac++) {
+                    const uint32_t n = fac ? n_f : n_v, big = fac ? nfb : nvb;
+                    for (uint32_t j = 0; j < (fac ? rf : rv); j++)
+                        for (uint32_t b = 0; b < nb; b++) {
+                            const uint32_t it = res_item_of(j, b, nb);
+                            if (it >= n) continue;
+                            uint32_t w;
+                            if (it < big) {
+                                w = fac ? L.fb_deg[L.nf_huge + it] : L.vb_deg[L.nv_huge + it];
+                            } else {
+                                const auto &gb = fac ? L.fg_base : L.vg_base;
+                                const uint32_t g = n - big - 1 - (it - big);
+                                w = (gb[g + 1] - gb[g]) >> 5;
+                            }
+                            words[b] += res_item_words(fac != 0, it < big, w, sizeof(T), batch);
+                        }
+                }
+                smem = 4 * (size_t)*std::max_element(words.begin(), words.end());
+                if (smem > kResSmemMax) continue;
+            }
+            const int bps = resident_blocks_per_sm<T>(damp, cache != 0, smem);
+            if ((uint64_t)bps * (uint64_t)e->sms < nb) continue;
+            e->res_plan = 1 + cache;
+            e->res_grid = nb;
+            e->res_rows_f = rf;
+            e->res_rows_v = rv;
+            e->res_smem = smem;
+            return;
+        }
+    }
+}
+
+// Whether runs of a mode take the resident kernel: the default forms, no
+// per-pass timing, a parallel schedule and a graph of its range.
+bool use_resident(flbp_engine *e, int mode) {
+    if (e->seq || e->ktime || e->f_form || e->v_form || e->L.V == 0 || e->n_sets) return false;
+    if (e->L.n_slots > (mode == 0 ? kResFixedSlots : kResRuleSlots)) return false;
+    if (e->res_plan < 0) {
+        if (e->prec == 64) plan_resident_t<double>(e);
+        else plan_resident_t<float>(e);
+    }
+    return e->res_plan > 0;
+}
+
+template <typename T>
+cudaError_t launch_resident_t(flbp_engine *e, int mode, uint32_t cap, bool final_beliefs) {
+    ResArgs<T> r;
+    r.f = factor_args<T>(e);
+    r.v = var_args(e);
+    if (mode == 3) {
+        r.f.f_graph = e->d_f_graph;
+        r.f.gdone = e->d_gstate;
+        r.v.v_graph = e->d_v_graph;
+        r.v.gstate = e->d_gstate;
+        r.f.n_graphs = r.v.n_graphs = e->n_graphs;
+    }
+    r.vf = (T *)e->d_vf;
+    r.fv = (T *)e->d_fv;
+    r.fvd = (T *)e->d_fvd;
+    r.d = (T)e->damping;
+    r.ctl = e->d_ctl;
+    r.cap = cap;
+    r.final_beliefs = final_beliefs ? 1 : 0;
+    r.rows_f = e->res_rows_f;
+    r.rows_v = e->res_rows_v;
+    return resident_launch<T>(e->damping != 0.0, e->res_plan == 2, e->res_grid, e->res_smem, r, e->stream);
+}
+
+// At most `cap` (<= kResSweeps) sweeps of a mode in one launch; `again`: not
+// the first launch after the control block's upload.
+int launch_resident(flbp_engine *e, int mode, long long cap, bool final_beliefs, bool again) {
+    if (again)
+        FLBP_CUDA(cudaMemsetAsync(reinterpret_cast<char *>(e->d_ctl) + offsetof(Ctl, rs), 0, sizeof(ResSync), e->stream));
+    FLBP_CUDA(e->prec == 64 ? launch_resident_t<double>(e, mode, (uint32_t)cap, final_beliefs)
+                            : launch_resident_t<float>(e, mode, (uint32_t)cap, final_beliefs));
+    e->launches += 1;
+    return FLBP_OK;
+}
+
 // Stop-rule driven loop: chunks of sweeps until the device sets ctl->done.
 int run_loop(flbp_engine *e, int mode, long long cap) {
     long long launched = 0;
+    if (use_resident(e, mode)) {
+        while (launched < cap) {
+            const long long n = std::min<long long>(kResSweeps, cap - launched);
+            int rc = launch_resident(e, mode, n, false, launched > 0);
+            if (rc || (rc = download_ctl(e))) return rc;
+            launched += n;
+            if (e->h_ctl->done) break;
+        }
+        return FLBP_OK;
+    }
     int k = 1;
     while (launched < cap) {
         const long long n = std::min<long long>(k, cap - launched);
@@ -1604,8 +1736,17 @@ int flbp_run_fixed(flbp_engine *e, int64_t sweeps, flbp_run_info *info) {
     }
     const long long l0 = e->launches;
     reset_ctl_for_run(e, 0);
-    if ((rc = record_start(e)) || (rc = upload_ctl(e)) || (rc = launch_sweeps(e, 0, sweeps))) return rc;
-    launch_beliefs_only(e, e->d_belief);
+    if ((rc = record_start(e)) || (rc = upload_ctl(e))) return rc;
+    if (sweeps > 0 && use_resident(e, 0)) {
+        for (long long left = sweeps; left > 0;) {
+            const long long n = std::min<long long>(kResSweeps, left);
+            if ((rc = launch_resident(e, 0, n, n == left, left < sweeps))) return rc;
+            left -= n;
+        }
+    } else {
+        if ((rc = launch_sweeps(e, 0, sweeps))) return rc;
+        launch_beliefs_only(e, e->d_belief);
+    }
     FLBP_CUDA(cudaMemcpyAsync(e->d_lowpass, e->d_belief, std::max<size_t>(1, e->L.V) * sizeof(double),
                               cudaMemcpyDeviceToDevice, e->stream));
     if ((rc = record_stop(e)) || (rc = download_ctl(e))) return rc;

@@ -34,6 +34,26 @@ namespace flbp {
 // Control block of one engine (device memory). Written by block 0 of the
 // factor pass (sweep counters, residual reset) and by the last block of the
 // variable pass (stop decision); read by every block at kernel entry.
+constexpr int kGroupWords = 128;  // groups that stop by themselves in one resident kernel, / 32
+
+// Grid-wide state of the resident run kernel (resident.cuh), zero before
+// each launch. Three slots in turn: sweep s uses slot s % 3 while block 0
+// clears the next one.
+struct ResSync {
+    unsigned int arrive;  // block arrivals at the barriers between the passes, over the whole launch
+    unsigned int pad[3];
+    // Per slot, one 16-byte word read at once by the barrier that ends a
+    // sweep: max |belief change| (double bits); blocks arrived, with
+    // kResTimeUp added once the run's time is over.
+    struct alignas(16) End {
+        unsigned long long maxdiff;
+        unsigned int arrive, pad;
+    } end[3];
+    unsigned long long nonconv[3];
+    unsigned int moved[3][kGroupWords];
+};
+constexpr unsigned int kResTimeUp = 1u << 24;
+
 struct Ctl {
     unsigned long long maxdiff_bits;  // max |belief change| of this sweep, double bits
     unsigned long long nonconv;       // variables with |belief change| > tol
@@ -60,6 +80,7 @@ struct Ctl {
     unsigned int fnext, vnext;        // next chunk of tiles of the factor / variable pass (reset by the other pass)
     // batched solves: number of tiles of the factor / variable pass that hold a live graph
     unsigned int n_act_f, n_act_v;
+    ResSync rs;
 };
 
 template <typename T>
@@ -103,6 +124,21 @@ __device__ __forceinline__ uint8_t ld_stream(const uint8_t *p) {
 }
 __device__ __forceinline__ float ld_stream(const float *p) { return __ldcs(p); }
 __device__ __forceinline__ double ld_stream(const double *p) { return __ldcs(p); }
+
+// A pointer whose reads come from L2: data that other SMs write while the
+// kernel runs.
+template <typename T>
+struct CgPtr {
+    const T *p;
+    __device__ __forceinline__ T operator[](uint32_t i) const { return __ldcg(p + i); }
+};
+
+// Element i of a message array: from L2 where other SMs write it while the
+// kernel runs (CG).
+template <bool CG, typename T>
+__device__ __forceinline__ T ld_msg(const T *p, uint32_t i) {
+    return CG ? __ldcg(p + i) : p[i];
+}
 
 // log(sigmoid(x)) = min(x,0) - log1p(exp(-|x|)); +inf -> 0, -inf -> -inf, NaN -> NaN.
 template <typename T>
@@ -278,6 +314,7 @@ struct AccOps<double> {
     static __device__ __forceinline__ void add(double &s, double x) { s += x; }
     static __device__ __forceinline__ void combine(double &s, double o) { s += o; }
     static __device__ __forceinline__ double value(double s) { return s; }
+    static __device__ __forceinline__ bool finite(double s) { return fabs(s) < Num<double>::inf(); }
     // s - x rounded once to the message type
     template <typename T>
     static __device__ __forceinline__ T excl(double s, T x) {
@@ -293,6 +330,7 @@ struct AccOps<float> {
     static __device__ __forceinline__ void add(float &s, float x) { s += x; }
     static __device__ __forceinline__ void combine(float &s, float o) { s += o; }
     static __device__ __forceinline__ double value(float s) { return (double)s; }
+    static __device__ __forceinline__ bool finite(float s) { return fabsf(s) < Num<float>::inf(); }
     template <typename T>
     static __device__ __forceinline__ T excl(float s, T x) {
         return (T)(s - (float)x);
@@ -314,6 +352,8 @@ struct AccOps<F2> {
         s.lo += o.lo;
     }
     static __device__ __forceinline__ double value(F2 s) { return (double)s.hi + (double)s.lo; }
+    // an infinite or NaN term leaves hi infinite or NaN
+    static __device__ __forceinline__ bool finite(F2 s) { return fabsf(s.hi) < Num<float>::inf(); }
     template <typename T>
     static __device__ __forceinline__ T excl(F2 s, T x) {
         return (T)((s.hi - (float)x) + s.lo);
@@ -770,8 +810,8 @@ __device__ __forceinline__ void warp_rscan_pairs(T &P, T &R, int lane) {
 //   (lanes before) o (own earlier slots) o (own later slots) o (lanes after),
 // from two shuffle scans over the lanes' pairs; no division, exact zeros
 // stay exact.
-template <typename T, int NV>
-__device__ __forceinline__ void factor_tile_big(const T *vb, const uint32_t *ps, uint32_t nbody, uint8_t kind, T p, T q,
+template <typename T, int NV, typename VB>
+__device__ __forceinline__ void factor_tile_big(VB vb, const uint32_t *ps, uint32_t nbody, uint8_t kind, T p, T q,
                                                 int lane, T *__restrict__ fv) {
     const T sgn = (kind & KIND_OR) ? T(-1) : T(1);
     const uint32_t k0 = (uint32_t)lane * NV;  // first body slot of this lane (body index)
@@ -847,9 +887,11 @@ __device__ __forceinline__ void factor_tile_big(const T *vb, const uint32_t *ps,
 // spread over all consumer threads of a block (called by all of them): a
 // log-sigmoid sum of the body (WideAcc) with a count of -inf terms, reduced
 // over the block in a fixed order, then every slot removes its own term.
-template <typename T>
-__device__ void factor_block_huge(const FactorArgs &a, uint32_t b, int tid, const T *__restrict__ vf,
-                                  T *__restrict__ fv, typename WideAcc<T>::type *s_l, int *s_nz) {
+constexpr uint32_t kHugeRegs = 4;
+
+template <typename T, typename VB>
+__device__ void factor_block_huge(const FactorArgs &a, uint32_t b, int tid, VB vf, T *__restrict__ fv,
+                                  typename WideAcc<T>::type *s_l, int *s_nz) {
     typedef typename WideAcc<T>::type A;
     typedef AccOps<A> O;
     const uint32_t fi = a.nf_sell + b;
@@ -863,10 +905,31 @@ __device__ void factor_block_huge(const FactorArgs &a, uint32_t b, int tid, cons
     const int lane = tid & 31, wid = tid >> 5;
     A L = O::zero();
     int nz = 0;
-    for (uint32_t k = s0 + 1 + tid; k < s1; k += kConsumers) {
-        const T ls = log_sigmoid<T>(s * vf[k]);
-        if (ls == -inf) nz++;
-        else O::add(L, ls);
+    // A thread's slots in rounds of kHugeRegs, whose loads are all in flight
+    // together; the log-sigmoids of the first round stay in registers.
+    constexpr uint32_t R = kHugeRegs;
+    const uint32_t body = s0 + 1, n = s1 - body;
+    T first[R];
+    for (uint32_t i0 = tid; i0 < n; i0 += R * kConsumers) {
+        T x[R];
+#pragma unroll
+        for (uint32_t u = 0; u < R; u++) {
+            const uint32_t i = i0 + u * kConsumers;
+            x[u] = i < n ? vf[body + i] : T(0);
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < R; u++) {
+            if (i0 + u * kConsumers < n) {
+                const T ls = log_sigmoid<T>(s * x[u]);
+                if (ls == -inf) nz++;
+                else O::add(L, ls);
+                x[u] = ls;
+            }
+        }
+        if (i0 == (uint32_t)tid) {
+#pragma unroll
+            for (uint32_t u = 0; u < R; u++) first[u] = x[u];
+        }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -888,23 +951,35 @@ __device__ void factor_block_huge(const FactorArgs &a, uint32_t b, int tid, cons
     if ((kind & HEAD_MASK) == HEAD_FREE && tid == 0)
         put_fv<T>(fv, a.f_pos[s0], s * head_out<T>(nz ? -inf : (T)O::value(L), p, q, Num<T>::log(p)));
     const BodyDen<T> D = body_den<T>(s * head_effective<T>(kind, vf[s0]), p, q);
-    for (uint32_t k = s0 + 1 + tid; k < s1; k += kConsumers) {
-        const T ls = log_sigmoid<T>(s * vf[k]);
+    auto send = [&](uint32_t e, T ls) {
         const bool z = (ls == -inf);
         const T lo = (nz - (int)z) ? -inf : (z ? (T)O::value(L) : O::template excl<T>(L, ls));
-        put_fv<T>(fv, a.f_pos[k], s * body_out<T>(lo, p, q, D));
+        put_fv<T>(fv, e, s * body_out<T>(lo, p, q, D));
+    };
+    for (uint32_t i0 = tid; i0 < n; i0 += R * kConsumers) {
+        uint32_t e[R];
+#pragma unroll
+        for (uint32_t u = 0; u < R; u++) {
+            const uint32_t i = i0 + u * kConsumers;
+            e[u] = i < n ? a.f_pos[body + i] : kSentinel;
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < R; u++) {
+            const uint32_t i = i0 + u * kConsumers;
+            if (i < n) send(e[u], i0 == (uint32_t)tid ? first[u] : log_sigmoid<T>(s * vf[body + i]));
+        }
     }
 }
 
 // Item `wid` of a staged big tile: dispatch on its body size.
-template <typename T>
-__device__ __forceinline__ void factor_tile_item(const T *vb, const uint32_t *ps, uint32_t deg, uint8_t kind, T p, T q,
+template <typename T, typename VB>
+__device__ __forceinline__ void factor_tile_item(VB vb, const uint32_t *ps, uint32_t deg, uint8_t kind, T p, T q,
                                                  int lane, T *__restrict__ fv) {
     const uint32_t nbody = deg - 1;
-    if (nbody <= 32) factor_tile_big<T, 1>(vb, ps, nbody, kind, p, q, lane, fv);
-    else if (nbody <= 64) factor_tile_big<T, 2>(vb, ps, nbody, kind, p, q, lane, fv);
-    else if (nbody <= 128) factor_tile_big<T, 4>(vb, ps, nbody, kind, p, q, lane, fv);
-    else factor_tile_big<T, 8>(vb, ps, nbody, kind, p, q, lane, fv);
+    if (nbody <= 32) factor_tile_big<T, 1, VB>(vb, ps, nbody, kind, p, q, lane, fv);
+    else if (nbody <= 64) factor_tile_big<T, 2, VB>(vb, ps, nbody, kind, p, q, lane, fv);
+    else if (nbody <= 128) factor_tile_big<T, 4, VB>(vb, ps, nbody, kind, p, q, lane, fv);
+    else factor_tile_big<T, 8, VB>(vb, ps, nbody, kind, p, q, lane, fv);
 }
 static_assert(kBigFactorBody == 256, "factor_tile_item covers bodies of up to 256 slots");
 
@@ -1108,48 +1183,140 @@ __device__ __forceinline__ T take_fv(T x, T old, T d) {
     return DAMP ? damp_mix(x, old, d) : x;
 }
 
+// The same for messages known to be finite.
+template <typename T, bool DAMP>
+__device__ __forceinline__ T take_fv_fin(T x, T old, T d) {
+    return DAMP ? fma(T(1) - d, x, d * old) : x;
+}
+
+// Finite (neither +-inf nor NaN).
+template <typename T>
+__device__ __forceinline__ bool is_fin(T x) {
+    return fabs(x) < Num<T>::inf();
+}
+
+// Sum of one sliced-ELL variable (one lane) whose new messages are x[0..w)
+// and previous damped ones xo: S, which comes in as the prior, plus the
+// messages in use, which replace x, with the +-inf counts added to the
+// prior's. As in var_warp_sum the messages are first taken as finite. w is
+// the group's width (the same on all lanes), at most W.
+template <typename T, int W, bool DAMP, typename A>
+__device__ __forceinline__ void var_lane_sum(uint32_t w, T *x, const T *xo, T d, A &S, int &npos, int &nneg) {
+    typedef AccOps<A> O;
+    const T inf = Num<T>::inf();
+    A F = S;
+#pragma unroll
+    for (int k = 0; k < W; k++)
+        if ((uint32_t)k < w) O::add(F, take_fv_fin<T, DAMP>(x[k], DAMP ? xo[k] : T(0), d));
+    if (O::finite(F)) {
+        S = F;
+        if (DAMP) {
+#pragma unroll
+            for (int k = 0; k < W; k++) x[k] = take_fv_fin<T, DAMP>(x[k], xo[k], d);
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < W; k++) {
+            if ((uint32_t)k < w) {
+                x[k] = take_fv<T, DAMP>(x[k], DAMP ? xo[k] : T(0), d);
+                if (x[k] == inf) npos++;
+                else if (x[k] == -inf) nneg++;
+                else O::add(S, x[k]);
+            }
+        }
+    }
+}
+
+// The leave-one-out messages of that variable to the slots en(k).
+template <typename T, int W, typename EN, typename A>
+__device__ __forceinline__ void var_lane_send(uint32_t w, const T *x, EN en, const A &S, int npos, int nneg,
+                                              T *__restrict__ vf) {
+    if (AccOps<A>::finite(S) && npos + nneg == 0) {  // then every message is finite
+#pragma unroll
+        for (int k = 0; k < W; k++) {
+            if ((uint32_t)k < w) {
+                const uint32_t e = en(k);
+                if (e != kSentinel) vf[e] = AccOps<A>::template excl<T>(S, x[k]);
+            }
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < W; k++) {
+            if ((uint32_t)k < w) {
+                const uint32_t e = en(k);
+                if (e != kSentinel) vf[e] = excl_msg<T>(S, npos, nneg, x[k]);
+            }
+        }
+    }
+}
+
+// Sum of one large variable over a warp (lane l takes entries l, l + 32,
+// ...): its prior plus the messages in use, with the +-inf counts. The
+// messages are first added as if all were finite; a sum that is finite then
+// was right, and only otherwise are the exact zeros counted apart. x(k) and
+// xo(k): new and previous damped message of entry k.
+template <typename T, bool DAMP, typename X, typename XO, typename A>
+__device__ __forceinline__ void var_warp_sum(X x, XO xo, uint32_t deg, const void *prior, uint32_t pidx, T d,
+                                             double pscale, int lane, A &S, int &npos, int &nneg) {
+    typedef AccOps<A> O;
+    A S0;
+    int p0, n0;
+    decode_prior<T>(prior, pidx, pscale, S0, p0, n0);
+    S = O::zero();
+    for (uint32_t k = lane; k < deg; k += 32) O::add(S, take_fv_fin<T, DAMP>(x(k), xo(k), d));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) O::combine(S, O::shfl_xor(S, o));
+    npos = p0;
+    nneg = n0;
+    if (!__all_sync(0xffffffffu, O::finite(S))) {
+        const T inf = Num<T>::inf();
+        int np = 0, nn = 0;
+        S = O::zero();
+        for (uint32_t k = lane; k < deg; k += 32) {
+            const T xv = take_fv<T, DAMP>(x(k), xo(k), d);
+            if (xv == inf) np++;
+            else if (xv == -inf) nn++;
+            else O::add(S, xv);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) O::combine(S, O::shfl_xor(S, o));
+        npos += __reduce_add_sync(0xffffffffu, np);
+        nneg += __reduce_add_sync(0xffffffffu, nn);
+    }
+    O::combine(S, S0);
+}
+
+// The leave-one-out messages of that variable to the slots en(k), and its
+// damped messages to fvd_run.
+template <typename T, bool DAMP, bool WRITE_VF, typename X, typename XO, typename EN, typename A>
+__device__ __forceinline__ void var_warp_send(X x, XO xo, EN en, T *fvd_run, uint32_t deg, T d, int lane, const A &S,
+                                              int npos, int nneg, T *__restrict__ vf) {
+    for (uint32_t k = lane; k < deg; k += 32) {
+        const T xv = take_fv<T, DAMP>(x(k), DAMP ? xo(k) : T(0), d);
+        if (DAMP) fvd_run[k] = xv;
+        if (WRITE_VF) {
+            const uint32_t e = en(k);
+            if (e != kSentinel) vf[e] = excl_msg<T>(S, npos, nneg, xv);
+        }
+    }
+}
+
 // One big variable of a staged big tile, one warp: its entries are en[k],
 // x[k] (and xo[k], the previous damped messages), k < deg, in the stage;
 // fvd_run is its run of damped messages in global memory.
 template <typename T, int BMODE, bool WRITE_VF, bool DAMP>
-__device__ __forceinline__ double var_tile_big(const VarArgs &a, uint32_t v, uint32_t deg, const uint32_t *en, T *x,
+__device__ __forceinline__ double var_tile_big(const VarArgs &a, uint32_t v, uint32_t deg, const uint32_t *en, const T *x,
                                                const T *xo, T *__restrict__ fvd_run, const void *prior, uint32_t pidx,
                                                int lane, T *__restrict__ vf, T d, double pscale, double tol,
                                                unsigned long long &cnt) {
     typedef typename WideAcc<T>::type A;
     typedef AccOps<A> O;
-    const T inf = Num<T>::inf();
-    A S = O::zero();
-    int npos = 0, nneg = 0;
-    for (uint32_t k = lane; k < deg; k += 32) {
-        T xv = x[k];
-        if (DAMP) {
-            xv = take_fv<T, DAMP>(xv, xo[k], d);
-            x[k] = xv;
-            fvd_run[k] = xv;
-        }
-        if (xv == inf) npos++;
-        else if (xv == -inf) nneg++;
-        else O::add(S, xv);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        O::combine(S, O::shfl_xor(S, o));
-        npos += __shfl_xor_sync(0xffffffffu, npos, o);
-        nneg += __shfl_xor_sync(0xffffffffu, nneg, o);
-    }
-    A S0;
-    int p0, n0;
-    decode_prior<T>(prior, pidx, pscale, S0, p0, n0);
-    O::combine(S, S0);
-    npos += p0;
-    nneg += n0;
-    if (WRITE_VF) {
-        for (uint32_t k = lane; k < deg; k += 32) {
-            const uint32_t e = en[k];
-            if (e != kSentinel) vf[e] = excl_msg<T>(S, npos, nneg, x[k]);
-        }
-    }
+    A S;
+    int npos, nneg;
+    var_warp_sum<T, DAMP>([&](uint32_t k) { return x[k]; }, [&](uint32_t k) { return DAMP ? xo[k] : T(0); }, deg, prior,
+                          pidx, d, pscale, lane, S, npos, nneg);
+    var_warp_send<T, DAMP, WRITE_VF>([&](uint32_t k) { return x[k]; }, [&](uint32_t k) { return DAMP ? xo[k] : T(0); },
+                                     [&](uint32_t k) { return en[k]; }, fvd_run, deg, d, lane, S, npos, nneg, vf);
     constexpr bool RESID = (BMODE == 1 || BMODE == 2 || BMODE == 4);
     return (lane == 0) ? var_finish<BMODE>(a, v, O::value(S), npos, nneg, tol, RESID ? a.belief[v] : 0.0, cnt) : 0.0;
 }
@@ -1159,8 +1326,8 @@ __device__ __forceinline__ double var_tile_big(const VarArgs &a, uint32_t v, uin
 // of them): a WideAcc sum with +-inf counts reduced over the block in a fixed
 // order, then every entry's leave-one-out message. Returns the belief change
 // on thread 0 (0 elsewhere).
-template <typename T, int BMODE, bool WRITE_VF, bool DAMP>
-__device__ double var_block_huge(const VarArgs &a, uint32_t b, int tid, const T *__restrict__ fv,
+template <typename T, int BMODE, bool WRITE_VF, bool DAMP, bool CG = false>
+__device__ double var_block_huge(const VarArgs &a, uint32_t b, int tid, const T *fv,
                                  T *__restrict__ vf, T *__restrict__ fvd, T d, double pscale, double tol,
                                  unsigned long long &cnt, typename WideAcc<T>::type *s_s, int *s_np, int *s_nn) {
     typedef typename WideAcc<T>::type A;
@@ -1173,7 +1340,7 @@ __device__ double var_block_huge(const VarArgs &a, uint32_t b, int tid, const T 
     A S = O::zero();
     int npos = 0, nneg = 0;
     for (uint32_t k = k0 + tid; k < k1; k += kConsumers) {
-        T x = fv[k];
+        T x = ld_msg<CG>(fv, k);
         if (DAMP) {
             x = take_fv<T, DAMP>(x, fvd[k], d);
             fvd[k] = x;
@@ -1211,7 +1378,7 @@ __device__ double var_block_huge(const VarArgs &a, uint32_t b, int tid, const T 
     if (WRITE_VF) {
         for (uint32_t k = k0 + tid; k < k1; k += kConsumers) {
             const uint32_t e = a.v_ent[k];
-            if (e != kSentinel) vf[e] = excl_msg<T>(S, npos, nneg, src[k]);
+            if (e != kSentinel) vf[e] = excl_msg<T>(S, npos, nneg, ld_msg<CG>(src, k));
         }
     }
     return (tid == 0) ? var_finish<BMODE>(a, v, O::value(S), npos, nneg, tol, RESID ? a.belief[v] : 0.0, cnt) : 0.0;
@@ -1490,7 +1657,7 @@ __global__ void __launch_bounds__(kBlockThreadsDev) var_pass_kernel(VarArgs a, c
                     const uint32_t base = gb[2 + wid] - gb[2];
                     const double dd = var_tile_big<T, BMODE, WRITE_VF, DAMP>(
                         a, v, reinterpret_cast<const uint32_t *>(st + VS::bold)[wid],
-                        reinterpret_cast<const uint32_t *>(st + VS::ent) + base, reinterpret_cast<T *>(st + VS::x) + base,
+                        reinterpret_cast<const uint32_t *>(st + VS::ent) + base, reinterpret_cast<const T *>(st + VS::x) + base,
                         reinterpret_cast<const T *>(st + VS::xo) + base, fvd + gb[2] + base, st + VS::prior, wid, lane,
                         vf, d, pscale, tol, cnt);
                     dmax = fmax(dmax, dd);
@@ -1501,39 +1668,55 @@ __global__ void __launch_bounds__(kBlockThreadsDev) var_pass_kernel(VarArgs a, c
                 const int w = (int)((gb[3 + wid] - gb[2 + wid]) >> 5);
                 const uint32_t t = 32u * wid + lane, v = 32u * gb[0] + t;
                 const uint32_t *en = reinterpret_cast<const uint32_t *>(st + VS::ent) + base;
-                T *x = reinterpret_cast<T *>(st + VS::x) + base;
+                const T *x = reinterpret_cast<const T *>(st + VS::x) + base;
                 const T *xo = reinterpret_cast<const T *>(st + VS::xo) + base;
                 const uint32_t g = a.v_graph ? reinterpret_cast<const uint32_t *>(st + VS::gid)[t] : 0;
                 const bool live = !(a.v_graph && graph_done(s_done, a.gstate, g));  // stopped graph: no work
                 const int wl = live ? w : 0;
                 typedef typename NarrowAcc<T>::type A;
-                A S = AccOps<A>::zero();
+                A S0 = AccOps<A>::zero();
                 int npos = 0, nneg = 0;
-                if (v < a.nv_sell) decode_prior<T>(st + VS::prior, t, pscale, S, npos, nneg);
-                for (int k = 0; k < wl; k++) {  // padding entries hold 0
+                if (v < a.nv_sell) decode_prior<T>(st + VS::prior, t, pscale, S0, npos, nneg);
+                // as if every message were finite (padding entries hold 0): a finite sum then was right
+                A S = S0;
+                for (int k = 0; k < wl; k++) {
                     const int i = 32 * k + lane;
-                    T xv = x[i];
-                    if (DAMP) {
-                        xv = take_fv<T, DAMP>(xv, xo[i], d);
-                        x[i] = xv;
-                        fvd[gb[2] + base + i] = xv;
+                    AccOps<A>::add(S, take_fv_fin<T, DAMP>(x[i], DAMP ? xo[i] : T(0), d));
+                }
+                if (AccOps<A>::finite(S) && npos + nneg == 0) {
+                    for (int k = 0; k < wl; k++) {
+                        const int i = 32 * k + lane;
+                        const T xv = take_fv_fin<T, DAMP>(x[i], DAMP ? xo[i] : T(0), d);
+                        if (DAMP) fvd[gb[2] + base + i] = xv;
+                        if (WRITE_VF) {
+                            const uint32_t e = en[i];
+                            if (e != kSentinel) vf[e] = AccOps<A>::template excl<T>(S, xv);
+                        }
                     }
-                    if (xv == inf) npos++;
-                    else if (xv == -inf) nneg++;
-                    else AccOps<A>::add(S, xv);
+                } else {  // exact zeros among the messages: counted apart
+                    S = S0;
+                    for (int k = 0; k < wl; k++) {
+                        const int i = 32 * k + lane;
+                        const T xv = take_fv<T, DAMP>(x[i], DAMP ? xo[i] : T(0), d);
+                        if (xv == inf) npos++;
+                        else if (xv == -inf) nneg++;
+                        else AccOps<A>::add(S, xv);
+                    }
+                    for (int k = 0; k < wl; k++) {
+                        const int i = 32 * k + lane;
+                        const T xv = take_fv<T, DAMP>(x[i], DAMP ? xo[i] : T(0), d);
+                        if (DAMP) fvd[gb[2] + base + i] = xv;
+                        if (WRITE_VF) {
+                            const uint32_t e = en[i];
+                            if (e != kSentinel) vf[e] = excl_msg<T>(S, npos, nneg, xv);
+                        }
+                    }
                 }
                 if (v < a.nv_sell && live) {
                     const double dd = var_finish<BMODE>(
                         a, v, AccOps<A>::value(S), npos, nneg, tol, RESID ? reinterpret_cast<const double *>(st + VS::bold)[t] : 0.0, cnt);
                     dmax = fmax(dmax, dd);
                     if (BMODE == 4 && dd > tol) mark_moved(s_moved, a, g);
-                }
-                if (WRITE_VF) {
-                    for (int k = 0; k < wl; k++) {
-                        const int i = 32 * k + lane;
-                        const uint32_t e = en[i];
-                        if (e != kSentinel) vf[e] = excl_msg<T>(S, npos, nneg, x[i]);
-                    }
                 }
             }
             __syncwarp();

@@ -1,0 +1,22 @@
+// Host launcher of the resident run kernel (resident.cu).
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include "resident.cuh"
+
+namespace flbp {
+
+constexpr size_t kResSmemMax = 214 * 1024;  // cached constants of a block at most (static shared memory beside them)
+
+// One cooperative launch of `grid` blocks with `smem` bytes of cached constants (cache).
+template <typename T>
+cudaError_t resident_launch(bool damp, bool cache, unsigned grid, size_t smem, const ResArgs<T> &a,
+                            cudaStream_t st);
+
+// Resident blocks per SM with `smem` bytes of dynamic shared memory; 0 when
+// the kernel cannot run so.
+template <typename T>
+int resident_blocks_per_sm(bool damp, bool cache, size_t smem);
+
+}  // namespace flbp
