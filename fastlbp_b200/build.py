@@ -20,8 +20,8 @@ INCLUDE = os.path.join(ROOT, "include")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libfastlbp_b200.so")
 
-SOURCES = ["engine.cu", "direct.cu", "resident.cu", "dlayout.cu", "layout.cpp", "model.cpp", "causal_bp.cpp", "fg_capi.cpp",
-           "noalloc.cu", "schedule.cpp"]
+SOURCES = ["engine.cu", "direct.cu", "resident.cu", "resident_cluster.cu", "dlayout.cu", "layout.cpp", "model.cpp",
+           "causal_bp.cpp", "fg_capi.cpp", "noalloc.cu", "schedule.cpp"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC = os.environ.get("NVCC", "nvcc")
 # -ftz=true: FP32 device arithmetic flushes subnormal results to zero (fewer instructions around the

@@ -55,7 +55,8 @@ __device__ __forceinline__ void factor_group_direct(const T *__restrict__ vf, co
     for (int k = 0; k < W; k++) x[k] = vf[base + 32u * k + lane];
 #pragma unroll
     for (int k = 0; k < W; k++) ps[k] = ld_stream(f_pos + base + 32u * k + lane);
-    if (deg > 0) factor_reg<T, W>([&](int k) { return x[k]; }, [&](int k) { return ps[k]; }, deg, kind, p, q, fv);
+    if (deg > 0) factor_reg<T, W>([&](int k) { return x[k]; }, [&](int k) { return ps[k]; }, deg, kind, p, q,
+                                     GlobalOut<T>{fv});
 }
 
 template <typename T>
@@ -148,7 +149,8 @@ __global__ void __launch_bounds__(kDirectThreads, MINB) factor_direct_kernel(Fac
         if (nx < n_items) hn = factor_item<T>(a, nx, nbig, lane);  // next header in flight during this item
         if (h.big) {
             if (h.live)
-                factor_tile_item<T>(vf + h.base, a.f_pos + h.base, h.end, h.kind, h.p, h.q, lane, fv);
+                factor_tile_item<T>(vf + h.base, a.f_pos + h.base, h.end, h.kind, h.p, h.q, lane,
+                                    GlobalOut<T>{fv});
         } else {
             factor_group_direct_w<T>((int)((h.end - h.base) >> 5), vf, a.f_pos, h.base, h.live ? h.deg : 0, h.kind,
                                      h.p, h.q, lane, fv);
@@ -195,7 +197,7 @@ __device__ __forceinline__ double var_group_direct(const VarArgs &a, const T *__
     double dd = 0.0;
     if (real) dd = var_finish<BMODE>(a, v, AccOps<A>::value(S), npos, nneg, tol, bold, cnt);
     if (WRITE_VF)
-        var_lane_send<T, W>(W, x, [&](int k) { return en[k]; }, S, npos, nneg, vf);
+        var_lane_send<T, W>(W, x, [&](int k) { return en[k]; }, S, npos, nneg, GlobalOut<T>{vf});
     return dd;
 }
 
@@ -232,7 +234,8 @@ __device__ __forceinline__ double var_warp_direct(const VarArgs &a, uint32_t b, 
     auto xo = [&](uint32_t k) { return DAMP ? fvd[k0 + k] : T(0); };
     var_warp_sum<T, DAMP>(x, xo, k1 - k0, a.prior, v, d, pscale, lane, S, npos, nneg);
     var_warp_send<T, DAMP, WRITE_VF>(x, xo, [&](uint32_t k) { return ld_stream(a.v_ent + k0 + k); },
-                                     DAMP ? fvd + k0 : nullptr, k1 - k0, d, lane, S, npos, nneg, vf);
+                                     DAMP ? fvd + k0 : nullptr, k1 - k0, d, lane, S, npos, nneg,
+                                     GlobalOut<T>{vf});
     return (lane == 0) ? var_finish<BMODE>(a, v, O::value(S), npos, nneg, tol, RESID ? a.belief[v] : 0.0, cnt) : 0.0;
 }
 

@@ -159,6 +159,21 @@ struct flbp_engine {
     unsigned res_grid = 1;
     uint32_t res_rows_f = 0, res_rows_v = 0;
     size_t res_smem = 0;
+    // Cluster run kernel: -1 not planned yet, 0 not for this engine, 1 planned;
+    // its cluster size, clusters, rows of items per block, shared memory, jobs
+    // (device) and position maps.
+    int cl_plan = -1;
+    unsigned cl_size = 1, cl_clusters = 1;
+    uint32_t cl_rows_f = 0, cl_rows_v = 0, cl_map_words = 0, cl_n_jobs = 0;
+    size_t cl_smem = 0;
+    bool cl_all = false;  // batches: every graph is one of its jobs
+    ClusterJob *d_cl_jobs = nullptr;
+    uint32_t *d_cl_map = nullptr;
+    double *d_gdiff = nullptr;           // per group: last belief change
+    std::vector<ClusterJob> batch_jobs;  // batches: every graph's items
+    std::vector<uint8_t> batch_huge;     // and whether it has items too large for a tile
+    uint32_t *d_cut_ent = nullptr;       // sets: cut entries as bits (per set)
+    uint32_t cut_words = 0;
     std::map<std::pair<int, int>, cudaGraphExec_t> graphs;  // (mode, sweeps) -> executable graph
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     float last_ms = 0.f;
@@ -854,13 +869,227 @@ cudaError_t launch_resident_t(flbp_engine *e, int mode, uint32_t cap, bool final
     return resident_launch<T>(e->damping != 0.0, e->res_plan == 2, e->res_grid, e->res_smem, r, e->stream);
 }
 
-// At most `cap` (<= kResSweeps) sweeps of a mode in one launch; `again`: not
-// the first launch after the control block's upload.
-int launch_resident(flbp_engine *e, int mode, long long cap, bool final_beliefs, bool again) {
+
+// ---- the cluster run kernel (resident_cluster.cuh)
+
+// Largest single graph that runs on one cluster, in device slots. Measured
+// per tolerance sweep against the resident kernel: FP32 6.1 : 9.3 us at 4 k
+// slots, 7.4 : 9.5 at 24 k, 9.7 : 10.2 at 40 k, 12.0 : 10.4 at 63 k; FP64
+// 10.1 : 11.4 at 12 k, 11.1 : 11.1 at 24 k, 15.6 : 11.6 at 40 k.
+constexpr uint64_t kClusterSlots32 = 42000, kClusterSlots64 = 18000;
+
+// Shared memory (bytes) of the fullest block when a cluster of nb blocks
+// holds a job with these tables of rows, or 0 when it is more than a block has.
+template <typename T>
+size_t cluster_job_smem(const HostLayout &L, const ClusterJob &J, uint32_t nb, uint32_t rf, uint32_t rv, bool damp) {
+    std::vector<size_t> words(nb, (3u * (rf + rv) + 31u) & ~31u);
+    for (int fac = 0; fac < 2; fac++) {
+        const uint32_t big = fac ? J.fb1 - J.fb0 : J.vb1 - J.vb0;
+        const uint32_t n = big + (fac ? J.fg1 - J.fg0 : J.vg1 - J.vg0);
+        const auto &gb = fac ? L.fg_base : L.vg_base;
+        for (uint32_t j = 0; j * nb < n; j++)
+            for (uint32_t b = 0; b < nb; b++) {
+                const uint32_t it = res_item_of(j, b, nb);
+                if (it >= n) continue;
+                uint32_t w;
+                if (it < big) {
+                    w = fac ? L.fb_deg[J.fb0 + it] : L.vb_deg[J.vb0 + it];
+                } else {
+                    const uint32_t g = (fac ? J.fg1 : J.vg1) - 1 - (it - big);
+                    w = (gb[g + 1] - gb[g]) >> 5;
+                }
+                words[b] += cluster_item_words(fac != 0, it < big, w, sizeof(T), damp);
+            }
+    }
+    const size_t bytes = 4 * *std::max_element(words.begin(), words.end());
+    return bytes <= kClusterSmemMax ? bytes : 0;
+}
+
+// Cluster size and jobs of this engine, or a plan of 0.
+template <typename T>
+int plan_cluster_t(flbp_engine *e) {
+    const HostLayout &L = e->L;
+    const bool damp = e->damping != 0.0;
+    e->cl_plan = 0;
+    std::vector<ClusterJob> all;
+    std::vector<uint8_t> huge;
+    if (e->n_graphs) {
+        all = e->batch_jobs;
+        huge = e->batch_huge;
+    } else {
+        if (!e->n_sets && L.n_slots > (sizeof(T) == 4 ? kClusterSlots32 : kClusterSlots64)) return FLBP_OK;
+        ClusterJob J = {};
+        J.fg1 = L.n_fgroups();
+        J.f_hi = L.nf_sell;
+        J.fb0 = L.nf_huge;
+        J.fb1 = L.nf_big;
+        J.vg1 = L.n_vgroups();
+        J.v_hi = L.nv_sell;
+        J.vb0 = L.nv_huge;
+        J.vb1 = L.nv_big;
+        all.assign(1, J);  // evidence sets: one job each, all alike
+        huge.assign(1, L.nf_huge || L.nv_huge);
+    }
+    const uint32_t copies = std::max<uint32_t>(1, e->n_sets);
+    auto items_f = [](const ClusterJob &J) { return J.fb1 - J.fb0 + J.fg1 - J.fg0; };
+    auto items_v = [](const ClusterJob &J) { return J.vb1 - J.vb0 + J.vg1 - J.vg0; };
+    auto job_slots = [&](const ClusterJob &J) {
+        return (uint64_t)(L.fg_base[J.fg1] - L.fg_base[J.fg0]) +
+               (J.fb1 > J.fb0 ? (uint64_t)(L.fb_off[J.fb1] - L.fb_off[J.fb0]) : 0u);
+    };
+    double best = 1e300;
+    std::vector<uint32_t> best_jobs;
+    for (uint32_t nb = 1; nb <= 16; nb *= 2) {
+        // the graphs that fit a cluster of this size, with the tables of the largest of them
+        std::vector<uint32_t> fit;
+        uint32_t rf = 0, rv = 0;
+        for (uint32_t k = 0; k < all.size(); k++) {
+            if (huge[k]) continue;
+            const uint32_t jf = (items_f(all[k]) + nb - 1) / nb, jv = (items_v(all[k]) + nb - 1) / nb;
+            if (!cluster_job_smem<T>(L, all[k], nb, jf, jv, damp)) continue;
+            fit.push_back(k);
+            rf = std::max(rf, jf);
+            rv = std::max(rv, jv);
+        }
+        size_t smem = 0;
+        std::vector<uint32_t> jobs;
+        for (uint32_t k : fit) {  // again with the common tables
+            const size_t b = cluster_job_smem<T>(L, all[k], nb, rf, rv, damp);
+            if (!b) continue;
+            smem = std::max(smem, b);
+            jobs.push_back(k);
+        }
+        if (jobs.empty()) continue;
+        const int nc = cluster_max_active<T>(damp, nb, smem);
+        if (nc < 1) continue;
+        // Estimated time of a sweep of everything (us). A job's sweep is its
+        // latency plus the messages a block sends, one store each at a rate
+        // that measured the same from 1 k to 10 k slots a block.
+        double longest = 0.0, total = 0.0, rest = 0.0;
+        std::vector<uint8_t> in(all.size(), 0);
+        for (uint32_t k : jobs) {
+            const double n = (double)job_slots(all[k]) / nb;
+            const double t = sizeof(T) == 4 ? 5.0 + 1.75e-3 * n : 8.0 + 3.0e-3 * n;
+            longest = std::max(longest, t);
+            total += t * copies;
+            in[k] = 1;
+        }
+        for (uint32_t k = 0; k < all.size(); k++)
+            if (!in[k]) rest += 1.2e-5 * (double)job_slots(all[k]);
+        const uint32_t nclusters = (uint32_t)std::min<uint64_t>((uint64_t)nc, (uint64_t)jobs.size() * copies);
+        if (e->n_sets) total = longest * ((copies + nclusters - 1) / nclusters) * nclusters;  // whole rounds of like jobs
+        const double t = std::max(longest, total / nclusters) + (rest > 0.0 ? 8.0 + rest : 0.0);
+        if (t >= best) continue;
+        best = t;
+        best_jobs = jobs;
+        e->cl_size = nb;
+        e->cl_clusters = nclusters;
+        e->cl_rows_f = rf;
+        e->cl_rows_v = rv;
+        e->cl_smem = smem;
+    }
+    if (best_jobs.empty()) return FLBP_OK;
+    // Few large evidence sets leave clusters idle; the direct form takes
+    // about 20 us and 16.5 us per million slots (48 sets of 158 k slots: 4.9 ms
+    // in either form, 8 of them 1.13 ms direct and 1.30 ms on clusters).
+    if (e->n_sets && best > 20.0 + 1.65e-5 * (double)L.n_slots * e->n_sets) return FLBP_OK;
+    // largest first
+    std::stable_sort(best_jobs.begin(), best_jobs.end(),
+                     [&](uint32_t x, uint32_t y) { return items_v(all[x]) > items_v(all[y]); });
+    std::vector<ClusterJob> jobs;
+    uint64_t half = 1;
+    for (uint32_t k : best_jobs) {
+        const ClusterJob &J = all[k];
+        const uint64_t sf = L.fg_base[J.fg1] - L.fg_base[J.fg0], sv = L.vg_base[J.vg1] - L.vg_base[J.vg0];
+        const uint64_t bf = J.fb1 > J.fb0 ? L.fb_off[J.fb1] - L.fb_off[J.fb0] : 0;
+        const uint64_t bv = J.vb1 > J.vb0 ? L.vb_off[J.vb1] - L.vb_off[J.vb0] : 0;
+        half = std::max(half, (std::max(sf + bf, sv + bv) + 3) / 4 + 1);
+        for (uint32_t c = 0; c < copies; c++) {
+            jobs.push_back(J);
+            if (e->n_sets) jobs.back().group = c;
+        }
+    }
+    e->cl_map_words = (uint32_t)(2 * half);
+    e->cl_n_jobs = (uint32_t)jobs.size();
+    e->cl_all = jobs.size() == all.size() * copies;
+    int rc;
+    const size_t groups = std::max<size_t>({1, e->n_sets, e->n_graphs});
+    if ((rc = dalloc(e, &e->d_cl_jobs, jobs.size())) || (rc = upload(e, e->d_cl_jobs, jobs)) ||
+        (rc = dalloc(e, &e->d_cl_map, (size_t)e->cl_map_words * e->cl_clusters)) || (rc = dalloc(e, &e->d_gdiff, groups)))
+        return rc;
+    FLBP_CUDA(cudaStreamSynchronize(e->stream));  // the job list is a local of this function
+    e->cl_plan = 1;
+    return FLBP_OK;
+}
+
+// Whether runs of a mode take the cluster kernel.
+int use_cluster(flbp_engine *e, int mode, bool *use) {
+    *use = false;
+    if (e->seq || e->ktime || e->f_form || e->v_form || e->L.V == 0) return FLBP_OK;
+    if ((e->n_sets || e->n_graphs) && mode != 3) return FLBP_OK;
+    if (e->cl_plan < 0)
+        if (int rc = e->prec == 64 ? plan_cluster_t<double>(e) : plan_cluster_t<float>(e)) return rc;
+    *use = e->cl_plan > 0;
+    return FLBP_OK;
+}
+
+template <typename T>
+cudaError_t launch_cluster_t(flbp_engine *e, int mode, uint32_t cap, bool final_beliefs) {
+    ClusterArgs<T> r;
+    r.f = factor_args<T>(e);
+    r.v = var_args(e);
+    r.groups = mode == 3;
+    r.sets = e->n_sets > 0;
+    if (mode == 3) {
+        r.v.gstate = e->d_gstate;
+        r.v.n_graphs = e->n_sets ? e->n_sets : e->n_graphs;
+    }
+    if (e->n_sets) {
+        r.v.set_vf_stride = e->set_vs;
+        r.v.set_fv_stride = e->set_es;
+        r.v.set_prior_stride = e->set_nv * (e->prec == 64 ? 16 : 8);
+        r.v.set_belief_stride = e->set_nv;
+    }
+    r.vf = (T *)e->d_vf;
+    r.fv = (T *)e->d_fv;
+    r.fvd = (T *)e->d_fvd;
+    r.d = (T)e->damping;
+    r.ctl = e->d_ctl;
+    r.jobs = e->d_cl_jobs;
+    r.n_jobs = e->cl_n_jobs;
+    r.map = e->d_cl_map;
+    r.map_words = e->cl_map_words;
+    r.cap = cap;
+    r.final_beliefs = final_beliefs ? 1 : 0;
+    r.rows_f = e->cl_rows_f;
+    r.rows_v = e->cl_rows_v;
+    r.gdiff = e->d_gdiff;
+    r.cut_ent = e->d_cut_ent;
+    r.cut_words = e->cut_words;
+    return cluster_launch<T>(e->damping != 0.0, e->cl_size, e->cl_clusters, e->cl_smem, r, e->stream);
+}
+
+// Kernels that run many sweeps in one launch, small graphs first: 2 the
+// cluster kernel, 1 the resident kernel, 0 neither.
+int run_kernel(flbp_engine *e, int mode, int *kind) {
+    bool cl = false;
+    if (int rc = use_cluster(e, mode, &cl)) return rc;
+    *kind = cl ? 2 : use_resident(e, mode) ? 1 : 0;
+    return FLBP_OK;
+}
+
+// At most `cap` (<= kResSweeps) sweeps of a mode in one launch of such a
+// kernel; `again`: not the first launch after the control block's upload.
+int launch_run(flbp_engine *e, int kind, int mode, long long cap, bool final_beliefs, bool again) {
     if (again)
         FLBP_CUDA(cudaMemsetAsync(reinterpret_cast<char *>(e->d_ctl) + offsetof(Ctl, rs), 0, sizeof(ResSync), e->stream));
-    FLBP_CUDA(e->prec == 64 ? launch_resident_t<double>(e, mode, (uint32_t)cap, final_beliefs)
-                            : launch_resident_t<float>(e, mode, (uint32_t)cap, final_beliefs));
+    const uint32_t n = (uint32_t)cap;
+    if (kind == 2)
+        FLBP_CUDA(e->prec == 64 ? launch_cluster_t<double>(e, mode, n, final_beliefs)
+                                : launch_cluster_t<float>(e, mode, n, final_beliefs));
+    else
+        FLBP_CUDA(e->prec == 64 ? launch_resident_t<double>(e, mode, n, final_beliefs)
+                                : launch_resident_t<float>(e, mode, n, final_beliefs));
     e->launches += 1;
     return FLBP_OK;
 }
@@ -868,10 +1097,13 @@ int launch_resident(flbp_engine *e, int mode, long long cap, bool final_beliefs,
 // Stop-rule driven loop: chunks of sweeps until the device sets ctl->done.
 int run_loop(flbp_engine *e, int mode, long long cap) {
     long long launched = 0;
-    if (use_resident(e, mode)) {
+    int kind = 0;
+    if (mode == 3) kind = use_resident(e, mode) ? 1 : 0;  // run_groups_tol has called the cluster kernel
+    else if (int rc = run_kernel(e, mode, &kind)) return rc;
+    if (kind) {
         while (launched < cap) {
             const long long n = std::min<long long>(kResSweeps, cap - launched);
-            int rc = launch_resident(e, mode, n, false, launched > 0);
+            int rc = launch_run(e, kind, mode, n, false, launched > 0);
             if (rc || (rc = download_ctl(e))) return rc;
             launched += n;
             if (e->h_ctl->done) break;
@@ -1499,6 +1731,47 @@ int create_engine(const flbp_graph_desc *graph, const flbp_engine_opts *opts, fl
         std::vector<uint32_t> fg(nf_pad, 0), vg(std::max<size_t>(1, nv_pad), 0);
         for (uint32_t f = 0; f < nf; f++) fg[f] = batch->factor_graph[L.factor_of_internal[f]];
         for (uint32_t iv = 0; iv < (uint32_t)L.V; iv++) vg[iv] = batch->var_graph[L.var_of_internal[iv]];
+        {  // every graph's items, for the cluster kernel
+            const uint32_t ng = e->n_graphs;
+            std::vector<ClusterJob> &J = e->batch_jobs;
+            J.assign(ng, ClusterJob{});
+            e->batch_huge.assign(ng, 0);
+            for (uint32_t f = 0; f < L.nf_sell; f++) {
+                ClusterJob &j = J[fg[f]];
+                if (j.f_hi == 0) j.f_lo = f;
+                j.f_hi = f + 1;
+            }
+            for (uint32_t v = 0; v < L.nv_sell; v++) {
+                ClusterJob &j = J[vg[v]];
+                if (j.v_hi == 0) j.v_lo = v;
+                j.v_hi = v + 1;
+            }
+            for (uint32_t b = 0; b < L.nf_big; b++) {
+                const uint32_t g = fg[L.nf_sell + b];
+                if (b < L.nf_huge) {
+                    e->batch_huge[g] = 1;
+                } else {
+                    if (J[g].fb1 == 0) J[g].fb0 = b;
+                    J[g].fb1 = b + 1;
+                }
+            }
+            for (uint32_t b = 0; b < L.nv_big; b++) {
+                const uint32_t g = vg[L.nv_sell + b];
+                if (b < L.nv_huge) {
+                    e->batch_huge[g] = 1;
+                } else {
+                    if (J[g].vb1 == 0) J[g].vb0 = b;
+                    J[g].vb1 = b + 1;
+                }
+            }
+            for (uint32_t g = 0; g < ng; g++) {
+                J[g].fg0 = J[g].f_lo / 32;
+                J[g].fg1 = (J[g].f_hi + 31) / 32;
+                J[g].vg0 = J[g].v_lo / 32;
+                J[g].vg1 = (J[g].v_hi + 31) / 32;
+                J[g].group = g;
+            }
+        }
         auto ranges = [](const hvec<uint32_t> &hdr, uint32_t nt) {
             std::vector<uint2> r(std::max<uint32_t>(1, nt));
             for (uint32_t t = 0; t < nt; t++)
@@ -1664,6 +1937,8 @@ int flbp_engine_destroy(flbp_engine *e) {
     for (void *b : e->d_in)
         if (b) cudaFree(b);
     if (e->d_set_cut) cudaFree(e->d_set_cut);
+    for (void *b : {(void *)e->d_cl_jobs, (void *)e->d_cl_map, (void *)e->d_gdiff, (void *)e->d_cut_ent})
+        if (b) cudaFree(b);
     for (void *b : {(void *)e->d_ftlist, (void *)e->d_ftoff, (void *)e->d_act_f, (void *)e->d_act_v,
                     (void *)e->d_act_flag, e->d_cub_tmp})
         if (b) cudaFree(b);
@@ -1737,10 +2012,12 @@ int flbp_run_fixed(flbp_engine *e, int64_t sweeps, flbp_run_info *info) {
     const long long l0 = e->launches;
     reset_ctl_for_run(e, 0);
     if ((rc = record_start(e)) || (rc = upload_ctl(e))) return rc;
-    if (sweeps > 0 && use_resident(e, 0)) {
+    int kind = 0;
+    if (sweeps > 0 && (rc = run_kernel(e, 0, &kind))) return rc;
+    if (kind) {
         for (long long left = sweeps; left > 0;) {
             const long long n = std::min<long long>(kResSweeps, left);
-            if ((rc = launch_resident(e, 0, n, n == left, left < sweeps))) return rc;
+            if ((rc = launch_run(e, kind, 0, n, n == left, left < sweeps))) return rc;
             left -= n;
         }
     } else {
@@ -2293,15 +2570,61 @@ static int run_groups_tol(flbp_engine *e, uint32_t G, double tol, int64_t maxite
     c.maxdiff = INFINITY;
     if ((rc = record_start(e))) return rc;
     long long done_sweeps = 0;
-    if (maxiter > 0 && maxtime > 0.0) {
-        if ((rc = upload_ctl(e)) || (rc = run_loop(e, 3, maxiter))) return rc;
-        if ((rc = download_ctl(e))) return rc;
-        done_sweeps = e->h_ctl->run_sweeps;
-    }
-    if ((rc = record_stop(e))) return rc;
     std::vector<int> st(4 * (size_t)G);
-    FLBP_CUDA(cudaMemcpyAsync(st.data(), e->d_gstate, st.size() * sizeof(int), cudaMemcpyDeviceToHost, e->stream));
-    FLBP_CUDA(cudaStreamSynchronize(e->stream));
+    auto fetch = [&]() -> int {
+        FLBP_CUDA(cudaMemcpyAsync(st.data(), e->d_gstate, st.size() * sizeof(int), cudaMemcpyDeviceToHost, e->stream));
+        FLBP_CUDA(cudaStreamSynchronize(e->stream));
+        return FLBP_OK;
+    };
+    if (maxiter > 0 && maxtime > 0.0) {
+        if ((rc = upload_ctl(e))) return rc;
+        bool cl = false, over = false, open = true;
+        if ((rc = use_cluster(e, 3, &cl))) return rc;
+        double cl_diff = 0.0;
+        long long cl_sweeps = 0;
+        if (cl) {  // the groups that fit a cluster, each to its own end
+            const auto began = std::chrono::steady_clock::now();
+            for (bool again = false; open && !over; again = true) {
+                if ((rc = launch_run(e, 2, 3, std::min<long long>(kResSweeps, maxiter), false, again)) ||
+                    (rc = download_ctl(e)) || (rc = fetch()))
+                    return rc;
+                over = e->h_ctl->done != 0;
+                std::vector<double> diff(G);
+                FLBP_CUDA(cudaMemcpy(diff.data(), e->d_gdiff, G * sizeof(double), cudaMemcpyDeviceToHost));
+                uint32_t n_open = 0;
+                cl_sweeps = 0;
+                cl_diff = 0.0;
+                for (uint32_t g = 0; g < G; g++) {
+                    const long long n = st[2 * (size_t)G + g];
+                    if (n && !st[g]) n_open++;
+                    if (n > cl_sweeps) cl_sweeps = n, cl_diff = diff[g];
+                    else if (n && n == cl_sweeps) cl_diff = std::max(cl_diff, diff[g]);
+                }
+                open = n_open > 0;
+            }
+            done_sweeps = cl_sweeps;
+            open = !e->cl_all;  // the other graphs follow, in the time that is left
+            if (open && !over) {
+                e->h_ctl->maxtime_ns -= (double)std::chrono::duration_cast<std::chrono::nanoseconds>(
+                                            std::chrono::steady_clock::now() - began).count();
+                std::memset(&e->h_ctl->rs, 0, sizeof(ResSync));
+                if ((rc = upload_ctl(e))) return rc;
+            }
+        }
+        if (open && !over) {
+            if ((rc = run_loop(e, 3, maxiter)) || (rc = download_ctl(e))) return rc;
+            done_sweeps = std::max<long long>(done_sweeps, e->h_ctl->run_sweeps);
+        }
+        if (cl) {
+            if ((rc = fetch())) return rc;
+            if (cl_sweeps > e->h_ctl->run_sweeps) e->h_ctl->maxdiff = cl_diff;
+            else if (cl_sweeps == e->h_ctl->run_sweeps) e->h_ctl->maxdiff = std::max(e->h_ctl->maxdiff, cl_diff);
+            bool all = true;
+            for (uint32_t g = 0; g < G; g++) all &= st[g] != 0;
+            e->h_ctl->reason = all ? FLBP_ALL_CONVERGED : FLBP_DIVERGED;
+        }
+    }
+    if ((rc = record_stop(e)) || (rc = fetch())) return rc;
     for (uint32_t g = 0; g < G; g++) {
         if (sweeps) sweeps[g] = st[2 * (size_t)G + g];
         if (reasons) reasons[g] = st[g] ? st[3 * (size_t)G + g] : FLBP_DIVERGED;
@@ -3318,6 +3641,12 @@ int flbp_sets_create(const flbp_graph_desc *graph, int64_t n_sets, const int64_t
         (!cut.empty() && ((rc = dalloc(e, &e->d_set_cut, cut.size())) || (rc = upload(e, e->d_set_cut, cut)))) ||
         (!slots.empty() && ((rc = dalloc(e, &e->d_set_slots, slots.size())) || (rc = upload(e, e->d_set_slots, slots)))))
         return fail(rc);
+    if (!cut.empty()) {  // the cut entries as bits, for the cluster kernel
+        e->cut_words = (uint32_t)((ne + 31) / 32);
+        std::vector<uint32_t> bits((size_t)S * e->cut_words, 0u);
+        for (const uint2 &c : cut) bits[(size_t)c.x * e->cut_words + (c.y >> 5)] |= 1u << (c.y & 31u);
+        if ((rc = dalloc(e, &e->d_cut_ent, bits.size())) || (rc = upload(e, e->d_cut_ent, bits))) return fail(rc);
+    }
     FLBP_CUDA(cudaMemsetAsync(e->d_belief, 0, S * nv_pad * sizeof(double), e->stream));
     FLBP_CUDA(cudaMemsetAsync(e->d_gstate, 0, 4 * sizeof(int) * S, e->stream));
     FLBP_CUDA(cudaStreamSynchronize(e->stream));

@@ -662,6 +662,16 @@ __device__ __forceinline__ void put_fv(T *__restrict__ fv, uint32_t e, T o) {
     if (e != kSentinel) fv[e] = o;
 }
 
+// Where an item's outputs go: position e of a global message array (other
+// sinks: resident_cluster.cuh).
+template <typename T>
+struct GlobalOut {
+    T *__restrict__ p;
+    __device__ __forceinline__ void operator()(uint32_t e, T o) const {
+        if (e != kSentinel) p[e] = o;
+    }
+};
+
 // Head output of an AND factor from the pair (P, R = 1 - P) of its whole
 // body: m1 ~ p P + q R, m0 ~ (1-p) P + (1-q) R (causal_bp_parall.cu:113-151
 // in log-odds). With q == 0 and P not a normal number, p P is taken in log
@@ -685,8 +695,10 @@ __device__ __forceinline__ T head_from_pair(T P, T R, T p, T q, LogP lP) {
 // 341-366 in log-odds; OR = AND on negated log-odds). Widths up to 8 keep
 // sigma, tau and the suffix pairs of every slot (4 W registers); wider
 // groups keep only the prefix pairs and evaluate sigma again on the way back.
-template <typename T, int W, typename VB, typename PS>
-__device__ __forceinline__ void factor_reg(VB vb, PS ps, int deg, uint8_t kind, T p, T q, T *__restrict__ fv) {
+// FLAT: the slots are evaluated without a branch per slot (padding slots
+// too), for callers with too few warps to hide the branches.
+template <typename T, int W, bool FLAT = false, typename VB, typename PS, typename OUT>
+__device__ __forceinline__ void factor_reg(VB vb, PS ps, int deg, uint8_t kind, T p, T q, OUT out) {
     const T sgn = (kind & KIND_OR) ? T(-1) : T(1);
     auto logP = [&]() {
         T l = T(0);
@@ -700,9 +712,8 @@ __device__ __forceinline__ void factor_reg(VB vb, PS ps, int deg, uint8_t kind, 
         T sg[W], ta[W];
 #pragma unroll
         for (int k = 1; k < W; k++) {
-            if (k < deg) {
-                sig_pair<T>(sgn * vb(k), sg[k], ta[k]);
-            } else {  // padding slot: the identity pair
+            if (FLAT || k < deg) sig_pair<T>(sgn * vb(k), sg[k], ta[k]);
+            if (k >= deg) {  // padding slot: the identity pair
                 sg[k] = T(1);
                 ta[k] = T(0);
             }
@@ -722,14 +733,22 @@ __device__ __forceinline__ void factor_reg(VB vb, PS ps, int deg, uint8_t kind, 
         T Pp = T(1), Rp = T(0);
 #pragma unroll
         for (int k = 1; k < W; k++) {
-            if (k < deg)
-                put_fv<T>(fv, ps(k), sgn * body_out_pr<T>(Pp * sP[k], fma(Pp, sR[k], Rp), p, q, D));
+            if (FLAT) {  // the outputs of all slots before the first store
+                sP[k] = sgn * body_out_pr<T>(Pp * sP[k], fma(Pp, sR[k], Rp), p, q, D);
+            } else if (k < deg) {
+                out(ps(k), sgn * body_out_pr<T>(Pp * sP[k], fma(Pp, sR[k], Rp), p, q, D));
+            }
             Rp = fma(Pp, ta[k], Rp);
             Pp = Pp * sg[k];
         }
+        if (FLAT) {
+#pragma unroll
+            for (int k = 1; k < W; k++)
+                if (k < deg) out(ps(k), sP[k]);
+        }
         // the head from the forward product, as in the wider form below, so that a
         // factor's outputs do not depend on the width of the group it lands in
-        if ((kind & HEAD_MASK) == HEAD_FREE) put_fv<T>(fv, ps(0), sgn * head_from_pair<T>(Pp, Rp, p, q, logP));
+        if ((kind & HEAD_MASK) == HEAD_FREE) out(ps(0), sgn * head_from_pair<T>(Pp, Rp, p, q, logP));
     } else {
         T pP[W], pR[W];
         T P = T(1), R = T(0);
@@ -744,7 +763,7 @@ __device__ __forceinline__ void factor_reg(VB vb, PS ps, int deg, uint8_t kind, 
                 P = P * sk;
             }
         }
-        if ((kind & HEAD_MASK) == HEAD_FREE) put_fv<T>(fv, ps(0), sgn * head_from_pair<T>(P, R, p, q, logP));
+        if ((kind & HEAD_MASK) == HEAD_FREE) out(ps(0), sgn * head_from_pair<T>(P, R, p, q, logP));
         const BodyDen<T> D = body_den<T>(lh, p, q);
         T Ps = T(1), Rs = T(0);
 #pragma unroll
@@ -752,7 +771,7 @@ __device__ __forceinline__ void factor_reg(VB vb, PS ps, int deg, uint8_t kind, 
             if (k < deg) {
                 T sk, tk;
                 sig_pair<T>(sgn * vb(k), sk, tk);
-                put_fv<T>(fv, ps(k), sgn * body_out_pr<T>(pP[k] * Ps, fma(pP[k], Rs, pR[k]), p, q, D));
+                out(ps(k), sgn * body_out_pr<T>(pP[k] * Ps, fma(pP[k], Rs, pR[k]), p, q, D));
                 Rs = fma(sk, Rs, tk);
                 Ps = sk * Ps;
             }
@@ -767,7 +786,7 @@ __device__ __forceinline__ void factor_group(int w, const T *vb, const uint32_t 
 #define FLBP_W(N) \
     case N:                                                                                           \
         factor_reg<T, N>([&](int k) { return vb[32 * k + lane]; }, [&](int k) { return ps[32 * k + lane]; }, deg, \
-                         kind, p, q, fv);                                                                     \
+                         kind, p, q, GlobalOut<T>{fv});                                                       \
         break;
         FLBP_W(2) FLBP_W(3) FLBP_W(4) FLBP_W(5) FLBP_W(6) FLBP_W(7) FLBP_W(8) FLBP_W(9) FLBP_W(10) FLBP_W(11)
         FLBP_W(12) FLBP_W(13) FLBP_W(14) FLBP_W(15) FLBP_W(16)
@@ -810,9 +829,9 @@ __device__ __forceinline__ void warp_rscan_pairs(T &P, T &R, int lane) {
 //   (lanes before) o (own earlier slots) o (own later slots) o (lanes after),
 // from two shuffle scans over the lanes' pairs; no division, exact zeros
 // stay exact.
-template <typename T, int NV, typename VB>
+template <typename T, int NV, typename VB, typename OUT>
 __device__ __forceinline__ void factor_tile_big(VB vb, const uint32_t *ps, uint32_t nbody, uint8_t kind, T p, T q,
-                                                int lane, T *__restrict__ fv) {
+                                                int lane, OUT out) {
     const T sgn = (kind & KIND_OR) ? T(-1) : T(1);
     const uint32_t k0 = (uint32_t)lane * NV;  // first body slot of this lane (body index)
     T sg[NV], ta[NV];
@@ -860,7 +879,7 @@ __device__ __forceinline__ void factor_tile_big(VB vb, const uint32_t *ps, uint3
             return nz ? -Num<T>::inf() : (T)O::value(l);
         };
         const T o = sgn * head_from_pair<T>(P, R, p, q, logP);
-        if (lane == 0) put_fv<T>(fv, ps[0], o);
+        if (lane == 0) out(ps[0], o);
     }
     const BodyDen<T> D = body_den<T>(sgn * head_effective<T>(kind, vh), p, q);
     // own later slots, then the lanes after: suffix pairs, backwards
@@ -877,7 +896,7 @@ __device__ __forceinline__ void factor_tile_big(VB vb, const uint32_t *ps, uint3
 #pragma unroll
     for (int u = 0; u < NV; u++) {
         if (k0 + u < nbody)
-            put_fv<T>(fv, ps[1 + k0 + u], sgn * body_out_pr<T>(Pp * sP[u], fma(Pp, sR[u], Rp), p, q, D));
+            out(ps[1 + k0 + u], sgn * body_out_pr<T>(Pp * sP[u], fma(Pp, sR[u], Rp), p, q, D));
         Rp = fma(Pp, ta[u], Rp);
         Pp = Pp * sg[u];
     }
@@ -972,14 +991,14 @@ __device__ void factor_block_huge(const FactorArgs &a, uint32_t b, int tid, VB v
 }
 
 // Item `wid` of a staged big tile: dispatch on its body size.
-template <typename T, typename VB>
+template <typename T, typename VB, typename OUT>
 __device__ __forceinline__ void factor_tile_item(VB vb, const uint32_t *ps, uint32_t deg, uint8_t kind, T p, T q,
-                                                 int lane, T *__restrict__ fv) {
+                                                 int lane, OUT out) {
     const uint32_t nbody = deg - 1;
-    if (nbody <= 32) factor_tile_big<T, 1, VB>(vb, ps, nbody, kind, p, q, lane, fv);
-    else if (nbody <= 64) factor_tile_big<T, 2, VB>(vb, ps, nbody, kind, p, q, lane, fv);
-    else if (nbody <= 128) factor_tile_big<T, 4, VB>(vb, ps, nbody, kind, p, q, lane, fv);
-    else factor_tile_big<T, 8, VB>(vb, ps, nbody, kind, p, q, lane, fv);
+    if (nbody <= 32) factor_tile_big<T, 1, VB, OUT>(vb, ps, nbody, kind, p, q, lane, out);
+    else if (nbody <= 64) factor_tile_big<T, 2, VB, OUT>(vb, ps, nbody, kind, p, q, lane, out);
+    else if (nbody <= 128) factor_tile_big<T, 4, VB, OUT>(vb, ps, nbody, kind, p, q, lane, out);
+    else factor_tile_big<T, 8, VB, OUT>(vb, ps, nbody, kind, p, q, lane, out);
 }
 static_assert(kBigFactorBody == 256, "factor_tile_item covers bodies of up to 256 slots");
 
@@ -1085,7 +1104,7 @@ __global__ void __launch_bounds__(kBlockThreadsDev) factor_pass_kernel(FactorArg
                 factor_tile_item<T>(reinterpret_cast<const T *>(st + FS::vbuf) + base,
                                     reinterpret_cast<const uint32_t *>(st + FS::pos) + base,
                                     reinterpret_cast<const uint32_t *>(st + FS::deg)[wid], st[FS::kind + wid],
-                                    pq[2 * wid], pq[2 * wid + 1], lane, fv);
+                                    pq[2 * wid], pq[2 * wid + 1], lane, GlobalOut<T>{fv});
             }
         } else if ((uint32_t)wid < gb[1]) {
             const uint32_t base = gb[2 + wid] - gb[2], f = 32u * wid + lane;
@@ -1228,24 +1247,17 @@ __device__ __forceinline__ void var_lane_sum(uint32_t w, T *x, const T *xo, T d,
 }
 
 // The leave-one-out messages of that variable to the slots en(k).
-template <typename T, int W, typename EN, typename A>
-__device__ __forceinline__ void var_lane_send(uint32_t w, const T *x, EN en, const A &S, int npos, int nneg,
-                                              T *__restrict__ vf) {
+template <typename T, int W, typename EN, typename A, typename OUT>
+__device__ __forceinline__ void var_lane_send(uint32_t w, const T *x, EN en, const A &S, int npos, int nneg, OUT out) {
     if (AccOps<A>::finite(S) && npos + nneg == 0) {  // then every message is finite
 #pragma unroll
         for (int k = 0; k < W; k++) {
-            if ((uint32_t)k < w) {
-                const uint32_t e = en(k);
-                if (e != kSentinel) vf[e] = AccOps<A>::template excl<T>(S, x[k]);
-            }
+            if ((uint32_t)k < w) out(en(k), AccOps<A>::template excl<T>(S, x[k]));
         }
     } else {
 #pragma unroll
         for (int k = 0; k < W; k++) {
-            if ((uint32_t)k < w) {
-                const uint32_t e = en(k);
-                if (e != kSentinel) vf[e] = excl_msg<T>(S, npos, nneg, x[k]);
-            }
+            if ((uint32_t)k < w) out(en(k), excl_msg<T>(S, npos, nneg, x[k]));
         }
     }
 }
@@ -1288,16 +1300,13 @@ __device__ __forceinline__ void var_warp_sum(X x, XO xo, uint32_t deg, const voi
 
 // The leave-one-out messages of that variable to the slots en(k), and its
 // damped messages to fvd_run.
-template <typename T, bool DAMP, bool WRITE_VF, typename X, typename XO, typename EN, typename A>
+template <typename T, bool DAMP, bool WRITE_VF, typename X, typename XO, typename EN, typename A, typename OUT>
 __device__ __forceinline__ void var_warp_send(X x, XO xo, EN en, T *fvd_run, uint32_t deg, T d, int lane, const A &S,
-                                              int npos, int nneg, T *__restrict__ vf) {
+                                              int npos, int nneg, OUT out) {
     for (uint32_t k = lane; k < deg; k += 32) {
         const T xv = take_fv<T, DAMP>(x(k), DAMP ? xo(k) : T(0), d);
         if (DAMP) fvd_run[k] = xv;
-        if (WRITE_VF) {
-            const uint32_t e = en(k);
-            if (e != kSentinel) vf[e] = excl_msg<T>(S, npos, nneg, xv);
-        }
+        if (WRITE_VF) out(en(k), excl_msg<T>(S, npos, nneg, xv));
     }
 }
 
@@ -1316,7 +1325,8 @@ __device__ __forceinline__ double var_tile_big(const VarArgs &a, uint32_t v, uin
     var_warp_sum<T, DAMP>([&](uint32_t k) { return x[k]; }, [&](uint32_t k) { return DAMP ? xo[k] : T(0); }, deg, prior,
                           pidx, d, pscale, lane, S, npos, nneg);
     var_warp_send<T, DAMP, WRITE_VF>([&](uint32_t k) { return x[k]; }, [&](uint32_t k) { return DAMP ? xo[k] : T(0); },
-                                     [&](uint32_t k) { return en[k]; }, fvd_run, deg, d, lane, S, npos, nneg, vf);
+                                     [&](uint32_t k) { return en[k]; }, fvd_run, deg, d, lane, S, npos, nneg,
+                                     GlobalOut<T>{vf});
     constexpr bool RESID = (BMODE == 1 || BMODE == 2 || BMODE == 4);
     return (lane == 0) ? var_finish<BMODE>(a, v, O::value(S), npos, nneg, tol, RESID ? a.belief[v] : 0.0, cnt) : 0.0;
 }

@@ -132,12 +132,13 @@ __device__ __forceinline__ void res_factor_group(uint32_t w, const T *vf, uint32
     if (CACHE) {
         if (deg > 0)
             factor_reg<T, W>([&](int k) { return x[k]; }, [&](int k) { return ps[32 * k + lane]; }, deg, kind, p, q,
-                             fv);
+                             GlobalOut<T>{fv});
     } else {
         uint32_t pr[W];
 #pragma unroll
         for (int k = 0; k < W; k++) pr[k] = (uint32_t)k < w ? __ldg(ps + 32 * k + lane) : kSentinel;
-        if (deg > 0) factor_reg<T, W>([&](int k) { return x[k]; }, [&](int k) { return pr[k]; }, deg, kind, p, q, fv);
+        if (deg > 0) factor_reg<T, W>([&](int k) { return x[k]; }, [&](int k) { return pr[k]; }, deg, kind, p, q,
+                                     GlobalOut<T>{fv});
     }
 }
 
@@ -174,7 +175,8 @@ __device__ __forceinline__ void res_var_group(uint32_t w, const T *fv, T *__rest
         for (int k = 0; k < W; k++)
             if ((uint32_t)k < w) fvd[base + 32u * k + lane] = x[k];
     }
-    var_lane_send<T, W>(w, x, [&](int k) { return CACHE ? ent[32 * k + lane] : en[k]; }, S, npos, nneg, vf);
+    var_lane_send<T, W>(w, x, [&](int k) { return CACHE ? ent[32 * k + lane] : en[k]; }, S, npos, nneg,
+                        GlobalOut<T>{vf});
 }
 
 // The whole run. CACHE: the block's items' constants in shared memory (else
@@ -326,7 +328,8 @@ __global__ void __launch_bounds__(kResThreads, sizeof(T) == 4 ? 2 : 1) resident_
                 if (batch && stopped(CACHE ? meta[32 + 64 * (sizeof(T) / 4)] : r.f.f_graph[fi])) continue;
                 const T *pq = CACHE ? reinterpret_cast<const T *>(meta + 32) : pqg + 2 * (size_t)fi;
                 factor_tile_item<T>(CgPtr<T>{vf + x.base}, CACHE ? sm + x.off : r.f.f_pos + x.base, x.w,
-                                    CACHE ? (uint8_t)(meta[0] >> 8) : r.f.f_kind[fi], pq[0], pq[1], lane, fv);
+                                    CACHE ? (uint8_t)(meta[0] >> 8) : r.f.f_kind[fi], pq[0], pq[1], lane,
+                                    GlobalOut<T>{fv});
             } else {
                 const uint32_t fi = 32u * (r.f.n_fgroups - 1 - (it - nfb)) + lane;
                 int deg;
@@ -413,7 +416,7 @@ __global__ void __launch_bounds__(kResThreads, sizeof(T) == 4 ? 2 : 1) resident_
                 auto old = [&](uint32_t k) { return DAMP ? fvd[k0 + k] : T(0); };
                 var_warp_sum<T, DAMP>(in, old, x.w, prior, pidx, r.d, pscale, lane, S, npos, nneg);
                 var_warp_send<T, DAMP, true>(in, old, [&](uint32_t k) { return ent[k]; }, DAMP ? fvd + k0 : nullptr,
-                                             x.w, r.d, lane, S, npos, nneg, vf);
+                                             x.w, r.d, lane, S, npos, nneg, GlobalOut<T>{vf});
                 Sv = AccOps<typename WideAcc<T>::type>::value(S);
             } else {
                 typedef typename NarrowAcc<T>::type A;

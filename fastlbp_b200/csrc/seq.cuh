@@ -130,7 +130,8 @@ __device__ __forceinline__ void seq_factor_item(const SeqArgs &a, uint32_t it, i
     __syncwarp();  // orders the v->f stores before the other lanes' loads
     const T *pq = reinterpret_cast<const T *>(a.pq);
     const T p = pq[2 * f], q = pq[2 * f + 1];
-    if (deg - 1 <= kBigFactorBody) factor_tile_item<T>(vf + s0, a.iota + s0, deg, kind, p, q, lane, nw);
+    if (deg - 1 <= kBigFactorBody) factor_tile_item<T>(vf + s0, a.iota + s0, deg, kind, p, q, lane,
+                                                              GlobalOut<T>{nw});
     else seq_factor_huge<T>(vf + s0, deg - 1, kind, p, q, lane, nw + s0);
     if ((kind & HEAD_MASK) != HEAD_FREE && lane == 0) nw[s0] = c;  // a clamped head's constant
 }

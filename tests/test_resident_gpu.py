@@ -12,7 +12,7 @@ groups.
 import numpy as np
 import pytest
 
-from fastlbp_b200 import BatchEngine, CausalFactorGraph, Engine, workloads
+from fastlbp_b200 import BatchEngine, CausalFactorGraph, Engine, SetsEngine, workloads
 from test_engine_gpu import _large_item_graph
 from test_forms_gpu import _with_isolated
 
@@ -110,4 +110,42 @@ def test_batch_equals_passes(prec, damping):
         one = e.run_batch_tol(1e-6, 25)
         got.append([e.beliefs(), *one, *e.fv_messages(), *e.vf_messages()])
     _equal(got[0], got[1], "batch")
+    e.close()
+
+
+@pytest.mark.parametrize("prec", [32, 64])
+@pytest.mark.parametrize("damping", [0.0, 0.2])
+def test_sets_equal_passes(prec, damping):
+    """Evidence sets taken by clusters (7 jobs of one graph, cut entries of large
+    variables among them) against the two-launch form."""
+    fl = workloads.config1(8, scale=0.003)
+    a = CausalFactorGraph.from_factors(fl).graph_arrays()
+    deg = np.bincount(a["slot_var"], minlength=a["n_vars"])
+    vs = np.argsort(-deg)[:12]
+    sets = [{int(v): int(v + k) % 2 for v in vs[:2 * k]} for k in range(7)]
+    got = []
+    for timed in (False, True):
+        e = SetsEngine(a, sets, precision=prec, damping=damping)
+        e.set_kernel_timing(timed)
+        e.init()
+        one = e.run_sets_tol(1e-6, 40)
+        got.append([e.beliefs(), *one])
+        e.close()
+    _equal(got[0], got[1], "sets")
+
+
+def test_batch_continued_and_limited():
+    """A second call continues from the first one's messages; a sweep limit ends some graphs."""
+    graphs = [_bingo(n, seed=n) for n in (20, 800, 90)]
+    e = BatchEngine(graphs, damping=0.1)
+    got = []
+    for timed in (False, True):
+        e.set_kernel_timing(timed)
+        e.reset_counts()
+        e.init()
+        one = e.run_batch_tol(1e-6, 9)
+        two = e.run_batch_tol(1e-5, 30)
+        info = e.info.as_dict()
+        got.append([*one, *two, e.beliefs(), [info["sweeps"], info["reason"], info["maxdiff"]], *e.vf_messages()])
+    _equal(got[0], got[1], "continued")
     e.close()
