@@ -508,7 +508,7 @@ def run_seq(args, rank, world, local):
     thread. Ours: FP32 and FP64 engines timed with CUDA events around
     run_fixed (kernels only, the graph resident), with the engine's choice of
     launch form and with each form forced (two launches per batch; the whole
-    sweep on one thread-block cluster). The reference's own code
+    sweep on one thread block). The reference's own code
     (oracle/_ref/ref_bp, REF_BP_UPDATES) runs the same schedule on the same
     graph in FP64, timed around its run(); its beliefs are compared with the
     FP64 engine's."""
@@ -530,9 +530,9 @@ def run_seq(args, rank, world, local):
         for prec in (32, 64):
             e = Engine(a, precision=prec, updates=updates)
             rec["batches"] = e.update_info()[1]
-            # 0: the engine's choice, 1: two launches per batch, 2: one cluster per sweep,
+            # 0: the engine's choice, 1: two launches per batch, 2: one block per sweep,
             # 3: two launches per batch with programmatic dependent launch
-            for kernel, tag in ((0, ""), (1, "_launches"), (2, "_cluster"), (3, "_pdl")):
+            for kernel, tag in ((0, ""), (1, "_launches"), (2, "_block"), (3, "_pdl")):
                 e.set_seq_kernel(kernel)
                 ts = []
                 for rep in range(max(1, args.warmup) + 2):

@@ -294,7 +294,7 @@ class Engine:
         check(lib().flbp_set_update_seq(self._h, sq.ctypes.data_as(C.c_void_p), sq.size))
 
     def set_seq_kernel(self, kind: int) -> None:
-        """Sequential sweeps: 0 choose, 1 two launches per batch, 2 one cluster
+        """Sequential sweeps: 0 choose, 1 two launches per batch, 2 one block
         per sweep, 3 as 1 with programmatic dependent launch
         (flbp_set_seq_kernel)."""
         check(lib().flbp_set_seq_kernel(self._h, int(kind)))
@@ -362,12 +362,12 @@ class Engine:
         return out
 
     def lowpass(self) -> np.ndarray:
-        out = np.zeros(self.n_vars)
+        out = np.empty(self.n_vars)
         check(lib().flbp_get_lowpass(self._h, out, out.size))
         return out
 
     def compute_beliefs(self) -> np.ndarray:
-        out = np.zeros(self.n_vars)
+        out = np.empty(self.n_vars)
         check(lib().flbp_compute_beliefs(self._h, out, out.size))
         return out
 
@@ -571,7 +571,9 @@ class SetsEngine(Engine):
         return sweeps, reasons
 
     def beliefs(self) -> np.ndarray:
-        out = np.zeros(self.n_sets * self.n_vars)
+        # not zeros(): large empty arrays come on huge pages, zeroed ones page by page
+        # (48 sets of 48 k variables: 3.9 ms to read out into zeros())
+        out = np.empty(self.n_sets * self.n_vars)
         check(lib().flbp_get_beliefs(self._h, out, out.size))
         return out.reshape(self.n_sets, self.n_vars)
 

@@ -551,11 +551,12 @@ __global__ void adjoint_prior_out_kernel(const T *__restrict__ gprior, const uin
     out_p[prior_factor[k]] += (double)gprior[prior_var[k]] * coef[k];
 }
 
-// Reference-order copy of an internal per-variable array.
-__global__ void gather_vars_kernel(const double *__restrict__ src, const uint32_t *__restrict__ internal_of_var,
-                                   int64_t n, double *__restrict__ out) {
+// Reference-order copies of gridDim.y internal per-variable arrays, `stride`
+// elements apart; output k at k n.
+__global__ void gather_vars_kernel(const double *__restrict__ src, uint64_t stride,
+                                   const uint32_t *__restrict__ internal_of_var, int64_t n, double *__restrict__ out) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = src[internal_of_var[i]];
+    if (i < n) out[(int64_t)blockIdx.y * n + i] = src[blockIdx.y * stride + internal_of_var[i]];
 }
 
 }  // namespace flbp

@@ -122,10 +122,10 @@ struct flbp_engine {
     bool seq = false;
     SeqLayout SQ;
     uint32_t *d_sq_foff = nullptr, *d_sq_var = nullptr, *d_sq_items = nullptr, *d_sq_tgt = nullptr;
-    uint32_t *d_sq_iota = nullptr, *d_sq_irec = nullptr, *d_sq_tvar = nullptr, *d_sq_bo = nullptr;
-    int seq_kernel = 0;        // 0: choose, 1: two launches per batch, 2: one cluster per sweep, 3: as 1 with
+    uint32_t *d_sq_iota = nullptr, *d_sq_irec = nullptr, *d_sq_tvar = nullptr, *d_sq_tst = nullptr, *d_sq_bo = nullptr;
+    int seq_kernel = 0;        // 0: choose, 1: two launches per batch, 2: one block per sweep, 3: as 1 with
                                // programmatic dependent launch
-    bool seq_cluster = false;  // the sweep runs as one cluster kernel
+    bool seq_block = false;  // the sweep runs as one launch on one block
     uint8_t *d_sq_kind = nullptr;
     void *d_sq_cst = nullptr, *d_sq_pq = nullptr, *d_sq_fv = nullptr, *d_sq_vf = nullptr, *d_sq_nw = nullptr;
     double *d_sq_S = nullptr;
@@ -277,6 +277,7 @@ SeqArgs seq_args(flbp_engine *e) {
     SeqArgs a;
     a.irec = reinterpret_cast<const uint4 *>(e->d_sq_irec);
     a.tvar = e->d_sq_tvar;
+    a.tst = e->d_sq_tst;
     a.bo = reinterpret_cast<const uint2 *>(e->d_sq_bo);
     a.foff = e->d_sq_foff;
     a.var = e->d_sq_var;
@@ -302,19 +303,20 @@ unsigned int seq_belief_grid(const flbp_engine *e) {
 // Kernels of one sequential sweep: `which` bit 0 the batches (with the
 // sweep's opening kernel), bit 1 the beliefs of the tolerance / low-pass loops.
 long long seq_sweep_launches(const flbp_engine *e, int mode, int which) {
-    const long long batches = e->seq_cluster ? 1 : 1 + 2LL * e->SQ.n_batches;
+    const long long batches = e->seq_block ? 1 : 1 + 2LL * e->SQ.n_batches;
     return ((which & 1) ? batches : 0) + (((which & 2) && (mode == 1 || mode == 2)) ? 1 : 0);
 }
 
-// One cluster per sweep where batches hold a few factors on average (TOPO's
-// hold two or three: a batch then takes 3.3 us on the cluster against 3.9 us
-// as two launches on a B200), else two launches per batch over the whole GPU
-// (SEQFIX's batches of a few hundred factors: 5.4 against 6.2 us).
-bool choose_seq_cluster(const flbp_engine *e) {
-    if (e->seq_kernel == 1 || e->seq_kernel == 3) return false;
-    if (e->seq_kernel == 2) return true;
+// One block per sweep where a batch's factors have few slots, else two
+// launches per batch over the whole GPU. Measured per batch, one block against
+// two launches: FP32 1.9 : 4.8 us at 42 slots a batch, 3.5 : 5.7 at 310, 6.1 :
+// 6.4 at 382 (with wide factors), 8.6 : 7.2 at 618; FP64 3.7 : 6.0 at 144,
+// 5.1 : 7.1 at 160, 7.7 : 6.7 at 244.
+bool choose_seq_block(const flbp_engine *e) {
     const SeqLayout &Q = e->SQ;
-    return Q.n_batches > 0 && Q.items.size() <= (size_t)Q.n_batches * 32;
+    if (e->seq_kernel == 1 || e->seq_kernel == 3 || Q.max_stage >= (1u << 24)) return false;
+    if (e->seq_kernel == 2) return true;
+    return Q.n_batches > 0 && (uint64_t)e->L.E <= (uint64_t)Q.n_batches * (e->prec == 64 ? 200 : 380);
 }
 
 // A kernel launch on the engine's stream, with programmatic dependent launch
@@ -338,13 +340,18 @@ void launch_seq_sweep(flbp_engine *e, int mode, int which) {
     const SeqArgs a = seq_args(e);
     const SeqLayout &Q = e->SQ;
     const bool pdl = (e->seq_kernel == 3);
-    if ((which & 1) && e->seq_cluster) {
-        if (e->damping != 0.0)
-            seq_sweep_cluster_kernel<T, true><<<kSeqClusterCtas, 32 * kSeqClusterWarps, 0, e->stream>>>(
-                a, Q.n_batches, (T)e->damping, e->d_ctl);
-        else
-            seq_sweep_cluster_kernel<T, false><<<kSeqClusterCtas, 32 * kSeqClusterWarps, 0, e->stream>>>(
-                a, Q.n_batches, (T)0, e->d_ctl);
+    if ((which & 1) && e->seq_block) {
+        const bool shared = Q.max_stage * sizeof(T) <= kSeqStageMax;
+        const size_t smem = shared ? Q.max_stage * sizeof(T) : 0;
+        const unsigned nt = 32 * kSeqBlockWarps<T>;
+        const T d = (T)e->damping;
+        auto go = [&](auto kern) {
+            if (smem > 48 * 1024)
+                cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSeqStageMax);
+            kern<<<1, nt, smem, e->stream>>>(a, Q.n_batches, shared ? 1 : 0, d, e->d_ctl);
+        };
+        if (e->damping != 0.0) go(seq_sweep_block_kernel<T, true>);
+        else go(seq_sweep_block_kernel<T, false>);
     } else if (which & 1) {
         launch_seq(e, pdl, seq_begin_kernel, 1, 1, e->d_ctl);
         const T d = (T)e->damping;
@@ -878,29 +885,54 @@ cudaError_t launch_resident_t(flbp_engine *e, int mode, uint32_t cap, bool final
 // 10.1 : 11.4 at 12 k, 11.1 : 11.1 at 24 k, 15.6 : 11.6 at 40 k.
 constexpr uint64_t kClusterSlots32 = 42000, kClusterSlots64 = 18000;
 
-// Shared memory (bytes) of the fullest block when a cluster of nb blocks
-// holds a job with these tables of rows, or 0 when it is more than a block has.
+// A job's items in shared-memory words: all of them, and the largest one.
+struct ClusterLoad {
+    uint64_t words = 0, largest = 0;
+};
 template <typename T>
-size_t cluster_job_smem(const HostLayout &L, const ClusterJob &J, uint32_t nb, uint32_t rf, uint32_t rv, bool damp) {
-    std::vector<size_t> words(nb, (3u * (rf + rv) + 31u) & ~31u);
-    for (int fac = 0; fac < 2; fac++) {
-        const uint32_t big = fac ? J.fb1 - J.fb0 : J.vb1 - J.vb0;
-        const uint32_t n = big + (fac ? J.fg1 - J.fg0 : J.vg1 - J.vg0);
-        const auto &gb = fac ? L.fg_base : L.vg_base;
+ClusterLoad cluster_load(const HostLayout &L, const ClusterJob &J, bool damp) {
+    ClusterLoad r;
+    auto add = [&](bool fac, bool big, uint32_t w) {
+        const uint64_t n = cluster_item_words(fac, big, w, sizeof(T), damp);
+        r.words += n;
+        r.largest = std::max(r.largest, n);
+    };
+    for (uint32_t b = J.fb0; b < J.fb1; b++) add(true, true, L.fb_deg[b]);
+    for (uint32_t b = J.vb0; b < J.vb1; b++) add(false, true, L.vb_deg[b]);
+    for (uint32_t g = J.fg0; g < J.fg1; g++) add(true, false, (L.fg_base[g + 1] - L.fg_base[g]) >> 5);
+    for (uint32_t g = J.vg0; g < J.vg1; g++) add(false, false, (L.vg_base[g + 1] - L.vg_base[g]) >> 5);
+    return r;
+}
+
+// Shared memory (bytes) that holds any block's share when a cluster of nb
+// blocks takes a job, or 0 when a block has less. Items are dealt row by row,
+// and within the large and the sliced-ELL items of a pass by decreasing size:
+// over the rows a block's share exceeds the mean by at most the largest item
+// for each of these four runs and for the row in which a pass changes from
+// one to the other. Where that bound is too much and the mean is not, the
+// shares are added up.
+template <typename T>
+size_t cluster_job_smem(const HostLayout &L, const ClusterJob &J, const ClusterLoad &w, uint32_t nb, uint32_t rf,
+                        uint32_t rv, bool damp) {
+    const uint64_t table = (3u * (rf + rv) + 31u) & ~31u, mean = (w.words + nb - 1) / nb;
+    const size_t bound = 4 * (table + mean + 6 * w.largest);
+    if (bound <= kClusterSmemMax) return bound;
+    if (4 * (table + mean) > kClusterSmemMax) return 0;
+    std::vector<uint64_t> words(nb, table);
+    auto deal = [&](bool fac, uint32_t b0, uint32_t b1, const hvec<uint32_t> &deg, uint32_t g0, uint32_t g1,
+                    const hvec<uint32_t> &base) {
+        const uint32_t big = b1 - b0, n = big + g1 - g0;
         for (uint32_t j = 0; j * nb < n; j++)
             for (uint32_t b = 0; b < nb; b++) {
                 const uint32_t it = res_item_of(j, b, nb);
                 if (it >= n) continue;
-                uint32_t w;
-                if (it < big) {
-                    w = fac ? L.fb_deg[J.fb0 + it] : L.vb_deg[J.vb0 + it];
-                } else {
-                    const uint32_t g = (fac ? J.fg1 : J.vg1) - 1 - (it - big);
-                    w = (gb[g + 1] - gb[g]) >> 5;
-                }
-                words[b] += cluster_item_words(fac != 0, it < big, w, sizeof(T), damp);
+                const uint32_t g = g1 - 1 - (it - big);
+                words[b] += it < big ? cluster_item_words(fac, true, deg[b0 + it], sizeof(T), damp)
+                                     : cluster_item_words(fac, false, (base[g + 1] - base[g]) >> 5, sizeof(T), damp);
             }
-    }
+    };
+    deal(true, J.fb0, J.fb1, L.fb_deg, J.fg0, J.fg1, L.fg_base);
+    deal(false, J.vb0, J.vb1, L.vb_deg, J.vg0, J.vg1, L.vg_base);
     const size_t bytes = 4 * *std::max_element(words.begin(), words.end());
     return bytes <= kClusterSmemMax ? bytes : 0;
 }
@@ -937,6 +969,9 @@ int plan_cluster_t(flbp_engine *e) {
         return (uint64_t)(L.fg_base[J.fg1] - L.fg_base[J.fg0]) +
                (J.fb1 > J.fb0 ? (uint64_t)(L.fb_off[J.fb1] - L.fb_off[J.fb0]) : 0u);
     };
+    std::vector<ClusterLoad> load(all.size());
+    for (size_t k = 0; k < all.size(); k++)
+        if (!huge[k]) load[k] = cluster_load<T>(L, all[k], damp);
     double best = 1e300;
     std::vector<uint32_t> best_jobs;
     for (uint32_t nb = 1; nb <= 16; nb *= 2) {
@@ -946,7 +981,7 @@ int plan_cluster_t(flbp_engine *e) {
         for (uint32_t k = 0; k < all.size(); k++) {
             if (huge[k]) continue;
             const uint32_t jf = (items_f(all[k]) + nb - 1) / nb, jv = (items_v(all[k]) + nb - 1) / nb;
-            if (!cluster_job_smem<T>(L, all[k], nb, jf, jv, damp)) continue;
+            if (!cluster_job_smem<T>(L, all[k], load[k], nb, jf, jv, damp)) continue;
             fit.push_back(k);
             rf = std::max(rf, jf);
             rv = std::max(rv, jv);
@@ -954,7 +989,7 @@ int plan_cluster_t(flbp_engine *e) {
         size_t smem = 0;
         std::vector<uint32_t> jobs;
         for (uint32_t k : fit) {  // again with the common tables
-            const size_t b = cluster_job_smem<T>(L, all[k], nb, rf, rv, damp);
+            const size_t b = cluster_job_smem<T>(L, all[k], load[k], nb, rf, rv, damp);
             if (!b) continue;
             smem = std::max(smem, b);
             jobs.push_back(k);
@@ -2142,7 +2177,15 @@ int flbp_run_lowpass(flbp_engine *e, double tol, int64_t min_iters, int64_t max_
 
 // A per-variable device array in the caller's variable order, gathered on
 // the device and copied straight into `out`.
-static int fetch_internal(flbp_engine *e, const double *dsrc, double *out, int64_t n) {
+//
+// `sets` consecutive such arrays (stride elements apart on the device) go
+// out one after the other: several per gather and copy, as many as the
+// staging of kFetchValues values holds. 48 sets of 48 k variables: 3.7 ms with
+// a gather, a copy and a wait per set.
+constexpr int64_t kFetchValues = 8 << 20;
+
+static int fetch_internal(flbp_engine *e, const double *dsrc, double *out, int64_t n, int64_t sets = 1,
+                          uint64_t stride = 0) {
     if (n != e->L.V) {
         set_error("output length must equal the number of variables");
         return FLBP_ERR_INVALID;
@@ -2153,14 +2196,19 @@ static int fetch_internal(flbp_engine *e, const double *dsrc, double *out, int64
         std::vector<uint32_t> iov(e->L.internal_of_var.begin(), e->L.internal_of_var.end());
         if ((rc = dalloc(e, &e->d_int_of_var, iov.size())) || (rc = upload(e, e->d_int_of_var, iov))) return rc;
     }
-    if (!e->d_ref_out && (rc = dalloc(e, &e->d_ref_out, (size_t)n))) return rc;
-    gather_vars_kernel<<<(unsigned)((n + 255) / 256), 256, 0, e->stream>>>(dsrc, e->d_int_of_var, n, e->d_ref_out);
-    e->launches += 1;
-    FLBP_CUDA(cudaGetLastError());
-    PinnedStage *S = n >= (1 << 16) ? stage_for(e->device) : nullptr;  // large outputs through the staging buffers
+    const int64_t per = std::min(sets, std::max<int64_t>(1, kFetchValues / n));
+    if (!e->d_ref_out && (rc = dalloc(e, &e->d_ref_out, (size_t)(per * n)))) return rc;
+    PinnedStage *S = per * n >= (1 << 16) ? stage_for(e->device) : nullptr;  // large outputs through the staging buffers
     std::unique_lock<std::mutex> lock;
     if (S) lock = std::unique_lock<std::mutex>(S->mu);
-    FLBP_CUDA(staged_d2h<double>(e, S, out, e->d_ref_out, (size_t)n));
+    for (int64_t k = 0; k < sets; k += per) {
+        const int64_t m = std::min(per, sets - k);
+        gather_vars_kernel<<<dim3((unsigned)((n + 255) / 256), (unsigned)m), 256, 0, e->stream>>>(
+            dsrc + (uint64_t)k * stride, stride, e->d_int_of_var, n, e->d_ref_out);
+        e->launches += 1;
+        FLBP_CUDA(cudaGetLastError());
+        FLBP_CUDA(staged_d2h<double>(e, S, out + k * n, e->d_ref_out, (size_t)(m * n)));
+    }
     return FLBP_OK;
 }
 
@@ -2173,9 +2221,7 @@ int flbp_get_beliefs(flbp_engine *e, double *out, int64_t n) {
             set_error("output length must equal the number of sets times the number of variables");
             return FLBP_ERR_INVALID;
         }
-        for (uint32_t k = 0; k < e->n_sets; k++)
-            if ((rc = fetch_internal(e, e->d_belief + (size_t)k * e->set_nv, out + (size_t)k * V, V))) return rc;
-        return FLBP_OK;
+        return fetch_internal(e, e->d_belief, out, V, (int64_t)e->n_sets, e->set_nv);
     }
     return fetch_internal(e, e->d_belief, out, n);
 }
@@ -3241,7 +3287,7 @@ int flbp_get_beliefs_device(flbp_engine *e, double *out, int64_t n) {
     }
     if (!e->d_int_of_var && (rc = ensure_adjoint_maps(e))) return rc;
     if (n) {
-        gather_vars_kernel<<<blocks_for(n, 256), 256, 0, e->stream>>>(e->d_belief, e->d_int_of_var, n, out);
+        gather_vars_kernel<<<blocks_for(n, 256), 256, 0, e->stream>>>(e->d_belief, 0, e->d_int_of_var, n, out);
         e->launches += 1;
     }
     FLBP_CUDA(cudaGetLastError());
@@ -3628,7 +3674,7 @@ int flbp_sets_create(const flbp_graph_desc *graph, int64_t n_sets, const int64_t
     }
     // S copies of the run state; the layout stays single
     for (void **b : {(void **)&e->d_vf, (void **)&e->d_fv, (void **)&e->d_fvd, (void **)&e->d_belief,
-                     (void **)&e->d_prior, (void **)&e->d_gstate})
+                     (void **)&e->d_prior, (void **)&e->d_gstate, (void **)&e->d_ref_out})
         if (*b) {
             dfree(e, *b);
             *b = nullptr;
@@ -3698,12 +3744,12 @@ namespace {
 void free_seq(flbp_engine *e) {
     void *bufs[] = {e->d_sq_foff, e->d_sq_var, e->d_sq_items, e->d_sq_tgt, e->d_sq_iota, e->d_sq_kind, e->d_sq_cst,
                     e->d_sq_pq,   e->d_sq_fv,  e->d_sq_vf,    e->d_sq_nw,  e->d_sq_S,    e->d_sq_cnt, e->d_sq_irec,
-                    e->d_sq_tvar, e->d_sq_bo};
+                    e->d_sq_tvar, e->d_sq_tst, e->d_sq_bo};
     for (void *b : bufs)
         dfree(e, b);
     e->d_sq_foff = e->d_sq_var = e->d_sq_items = e->d_sq_tgt = e->d_sq_iota = nullptr;
-    e->d_sq_irec = e->d_sq_tvar = e->d_sq_bo = nullptr;
-    e->seq_cluster = false;
+    e->d_sq_irec = e->d_sq_tvar = e->d_sq_tst = e->d_sq_bo = nullptr;
+    e->seq_block = false;
     e->d_sq_kind = nullptr;
     e->d_sq_cst = e->d_sq_pq = e->d_sq_fv = e->d_sq_vf = e->d_sq_nw = nullptr;
     e->d_sq_S = nullptr;
@@ -3782,6 +3828,7 @@ int flbp_set_update_seq(flbp_engine *e, const int64_t *seq, int64_t n) {
             (rc = dalloc(e, &e->d_sq_iota, ne)) || (rc = upload(e, e->d_sq_iota, iota)) ||
             (rc = dalloc(e, &e->d_sq_irec, S.irec.size())) || (rc = upload(e, e->d_sq_irec, S.irec)) ||
             (rc = dalloc(e, &e->d_sq_tvar, S.tvar.size())) || (rc = upload(e, e->d_sq_tvar, S.tvar)) ||
+            (rc = dalloc(e, &e->d_sq_tst, S.tst.size())) || (rc = upload(e, e->d_sq_tst, S.tst)) ||
             (rc = dalloc(e, &e->d_sq_bo, S.bo.size())) || (rc = upload(e, e->d_sq_bo, S.bo)) ||
             (rc = dalloc(e, &e->d_sq_S, nv)) || (rc = dalloc(e, &e->d_sq_cnt, nv)) ||
             (rc = (e->prec == 64 ? upload_seq_consts<double>(e) : upload_seq_consts<float>(e)))) {
@@ -3789,7 +3836,7 @@ int flbp_set_update_seq(flbp_engine *e, const int64_t *seq, int64_t n) {
             return rc;
         }
         e->seq = true;
-        e->seq_cluster = choose_seq_cluster(e);
+        e->seq_block = choose_seq_block(e);
     }
     if ((rc = flbp_init(e))) return rc;
     FLBP_CUDA(cudaStreamSynchronize(e->stream));
@@ -3800,7 +3847,7 @@ int flbp_set_seq_kernel(flbp_engine *e, int32_t kind) {
     int rc = begin_call(e);
     if (rc) return rc;
     if (kind < 0 || kind > 3) {
-        set_error("kind must be 0 (choose), 1 (two launches per batch), 2 (one cluster per sweep) or 3 (two "
+        set_error("kind must be 0 (choose), 1 (two launches per batch), 2 (one block per sweep) or 3 (two "
                   "launches per batch with programmatic dependent launch)");
         return FLBP_ERR_INVALID;
     }
@@ -3808,7 +3855,7 @@ int flbp_set_seq_kernel(flbp_engine *e, int32_t kind) {
     for (auto &kv : e->graphs) cudaGraphExecDestroy(kv.second);
     e->graphs.clear();
     e->seq_kernel = kind;
-    e->seq_cluster = e->seq && choose_seq_cluster(e);
+    e->seq_block = e->seq && choose_seq_block(e);
     return FLBP_OK;
 }
 

@@ -201,8 +201,10 @@ struct SeqLayout {
     hvec<double> pq;       // per reference factor: p, q
     hvec<uint32_t> ioff, items;  // per batch: its factors
     hvec<uint32_t> toff, tgt;    // per batch: its target device slots
-    hvec<uint32_t> irec;         // per item: first device slot, degree, kind, factor (4 words)
+    hvec<uint32_t> irec;         // per item: first device slot, degree, kind | staging offset << 8, factor (4 words)
     hvec<uint32_t> tvar;         // per target: its internal variable
+    hvec<uint32_t> tst;          // per target: staging offset of its message in its batch
+    uint64_t max_stage = 0;      // slots of the factors of the largest batch (offsets fit from 2^24 down)
     hvec<uint32_t> bo;           // per batch and the end: first item, first target (2 words)
 };
 

@@ -241,11 +241,31 @@ int build_seq_layout(const flbp_graph_desc &g, const HostLayout &L, const int64_
         const uint32_t I = S.items[it];
         S.irec[4 * it] = S.foff[I];
         S.irec[4 * it + 1] = S.foff[I + 1] - S.foff[I];
-        S.irec[4 * it + 2] = S.kind[I];
+        S.irec[4 * it + 2] = S.kind[I];  // staging offset above it, below
         S.irec[4 * it + 3] = I;
     }
     S.tvar.resize((size_t)E);
     for (int64_t k = 0; k < E; k++) S.tvar[k] = S.var[S.tgt[k]];
+    // The outputs of a batch are staged item after item: offset of every item
+    // (24 bits beside its kind) and of every target's message.
+    S.tst.resize((size_t)E);
+    S.max_stage = 0;
+    {
+        std::vector<uint64_t> at((size_t)F, 0);  // staging offset of the factors of the current batch
+        for (uint32_t b = 0; b < nb; b++) {
+            uint64_t n = 0;
+            for (uint32_t it = S.ioff[b]; it < S.ioff[b + 1]; it++) {
+                at[S.irec[4 * it + 3]] = n;
+                S.irec[4 * it + 2] |= (uint32_t)(n << 8);
+                n += S.irec[4 * it + 1];
+            }
+            for (uint32_t k = S.toff[b]; k < S.toff[b + 1]; k++) {
+                const uint32_t I = fos[S.tgt[k]];  // a factor's device slots are its reference slots, head first
+                S.tst[k] = (uint32_t)(at[I] + (S.tgt[k] - S.foff[I]));
+            }
+            S.max_stage = std::max(S.max_stage, n);
+        }
+    }
     S.bo.resize(2 * ((size_t)nb + 1));
     for (uint32_t b = 0; b <= nb; b++) {
         S.bo[2 * b] = S.ioff[b];
