@@ -76,21 +76,19 @@ __global__ void k_validate(DevGraphIn in, int64_t V, int64_t F, int64_t E, unsig
     }
 }
 
-// Sort key of an active factor: sliced-ELL ones by degree, within a degree
-// the ones that are not linked in index order, then the linked ones by the
-// degree class of their OR factor and their slot in it (layout.cpp); then
-// the large ones, too large for a tile first, by decreasing degree; inactive
-// factors last. 42 bits.
-constexpr int kFactorKeyBits = 42;
+// Sort key of an active factor: sliced-ELL ones by degree, then the large
+// ones, too large for a tile first, by decreasing degree; inactive factors
+// last. 38 bits.
+constexpr int kFactorKeyBits = 38;
 constexpr uint64_t kInactiveKey = (1ull << kFactorKeyBits) - 1;
 
 // Active / head state / constant message of every factor (the host's
 // classify_factor: +-det_logit(p) of singletons and of unclamped factors of
-// one slot, +-inf of clamped heads) and counts: cnt[0] sliced-ELL factors,
-// cnt[1] large ones, cnt[2] slots of active factors. Per variable the number
-// of its entries and the exclusive-or of their (factor, slot) pairs.
+// one slot, +-inf of clamped heads), the factor sort keys and counts:
+// cnt[0] sliced-ELL factors, cnt[1] large ones, cnt[2] slots of active
+// factors.
 __global__ void k_classify(DevGraphIn in, int64_t F, uint8_t *active, uint8_t *hstate, double *fconst,
-                           uint32_t *n_ent, unsigned long long *ends, unsigned long long *cnt) {
+                           uint64_t *fkey, uint32_t *fidx, unsigned long long *cnt) {
     const double inf = __longlong_as_double(0x7ff0000000000000ll);
     unsigned long long n_sell = 0, n_big = 0, n_slots = 0;
     GS_LOOP(i, F) {
@@ -115,51 +113,24 @@ __global__ void k_classify(DevGraphIn in, int64_t F, uint8_t *active, uint8_t *h
         active[I] = act;
         hstate[I] = hs;
         fconst[I] = c;
+        fidx[I] = (uint32_t)I;
+        uint64_t key = kInactiveKey;
         if (act) {
-            if (d <= (int64_t)kSellFactorDegree) n_sell++;
-            else n_big++;
-            n_slots += (unsigned long long)d;
-            const int64_t h = in.head[I];
-            for (int64_t e = in.off[I]; e < in.off[I + 1]; e++) {
-                if (e == h && hs != HEAD_FREE) continue;
-                const uint32_t v = (uint32_t)in.slot_var[e];
-                atomicAdd(&n_ent[v], 1u);
-                atomicXor(&ends[v], (unsigned long long)I << 32 | (unsigned long long)e);
+            if (d <= (int64_t)kSellFactorDegree) {
+                key = (uint64_t)d << 33;
+                n_sell++;
+            } else {
+                const uint64_t huge = (uint64_t)(d - 1 > (int64_t)kBigFactorBody ? 0 : 1);
+                key = (17ull << 33) | (huge << 32) | (uint64_t)(0xffffffffu - (uint32_t)d);
+                n_big++;
             }
+            n_slots += (unsigned long long)d;
         }
+        fkey[I] = key;
     }
     warp_add(&cnt[0], n_sell);
     warp_add(&cnt[1], n_big);
     warp_add(&cnt[2], n_slots);
-}
-
-// The factor sort keys.
-__global__ void k_factor_keys(DevGraphIn in, int64_t F, const uint8_t *active, const uint8_t *hstate,
-                              const uint32_t *n_ent, const unsigned long long *ends, uint64_t *fkey, uint32_t *fidx) {
-    GS_LOOP(i, F) {
-        const int64_t I = (int64_t)i;
-        const int64_t d = in.off[I + 1] - in.off[I];
-        uint64_t key = kInactiveKey;
-        if (active[I] && d <= (int64_t)kSellFactorDegree) {
-            key = (uint64_t)d << 37;
-            const int64_t h = in.head[I];
-            const uint32_t v = (uint32_t)in.slot_var[h];
-            if (in.type[I] == FLBP_AND && hstate[I] == HEAD_FREE && n_ent[v] == 2) {
-                const unsigned long long o = ends[v] ^ ((unsigned long long)I << 32 | (unsigned long long)h);
-                const int64_t J = (int64_t)(o >> 32), e = (int64_t)(o & 0xffffffffull);
-                if (J != I && in.type[J] == FLBP_OR && (int64_t)in.head[J] != e) {
-                    const int64_t dj = in.off[J + 1] - in.off[J];
-                    const uint64_t c = (uint64_t)(dj <= (int64_t)kSellFactorDegree ? dj : (int64_t)kSellFactorDegree + 1);
-                    key |= c << 32 | (uint64_t)e;
-                }
-            }
-        } else if (active[I]) {
-            const uint64_t huge = (uint64_t)(d - 1 > (int64_t)kBigFactorBody ? 0 : 1);
-            key = (17ull << 37) | (huge << 32) | (uint64_t)(0xffffffffu - (uint32_t)d);
-        }
-        fkey[I] = key;
-        fidx[I] = (uint32_t)I;
-    }
 }
 
 // Per active factor in internal order: kind, (p, q), degree; large ones'
@@ -222,10 +193,11 @@ __global__ void k_dev_slot(DevGraphIn in, const uint32_t *foi, uint32_t nf, uint
 }
 
 // Entries: every slot of an active factor reaches its variable, except a
-// clamped head. Entry flags of the reference slots, the variable of each
-// device slot, and every variable's first device slot.
+// clamped head. Entry flags of the reference slots, variable degrees, the
+// variable of each device slot, and every variable's first device slot.
 __global__ void k_entries(DevGraphIn in, const uint32_t *foi, uint32_t nf, const uint8_t *hstate,
-                          const uint32_t *dev_slot, uint8_t *is_entry, uint32_t *var_of_dev, uint32_t *first) {
+                          const uint32_t *dev_slot, uint8_t *is_entry, uint32_t *vdeg, uint32_t *var_of_dev,
+                          uint32_t *first) {
     GS_LOOP(f, nf) {
         const uint32_t I = foi[f];
         const int64_t h = in.head[I];
@@ -233,6 +205,7 @@ __global__ void k_entries(DevGraphIn in, const uint32_t *foi, uint32_t nf, const
             if (e == h && hstate[I] != HEAD_FREE) continue;
             const uint32_t v = (uint32_t)in.slot_var[e];
             is_entry[e] = 1;
+            atomicAdd(&vdeg[v], 1u);
             var_of_dev[dev_slot[e]] = v;
             atomicMin(&first[v], dev_slot[e]);
         }
@@ -549,15 +522,7 @@ int build_layout_device(const flbp_graph_desc &g, const DevGraphIn &in, int prec
     unsigned long long *cnt = P.get<unsigned long long>(4);
     DL_CHECK(P.err);
     DL_CHECK(cudaMemsetAsync(cnt, 0, 4 * sizeof(unsigned long long), st));
-    uint32_t *n_ent_of = P.get<uint32_t>(V);
-    unsigned long long *ends_of = P.get<unsigned long long>(V);
-    DL_CHECK(P.err);
-    DL_CHECK(cudaMemsetAsync(n_ent_of, 0, std::max<int64_t>(1, V) * 4, st));
-    DL_CHECK(cudaMemsetAsync(ends_of, 0, std::max<int64_t>(1, V) * 8, st));
-    if (F > 0) {
-        k_classify<<<grid_for(F), kTPB, 0, st>>>(in, F, active, hstate, fconst, n_ent_of, ends_of, cnt);
-        k_factor_keys<<<grid_for(F), kTPB, 0, st>>>(in, F, active, hstate, n_ent_of, ends_of, fkey, fidx);
-    }
+    if (F > 0) k_classify<<<grid_for(F), kTPB, 0, st>>>(in, F, active, hstate, fconst, fkey, fidx, cnt);
     if (F > 0) DL_CHECK(sort_pairs(fkey, fkey2, fidx, foi, (size_t)F, kFactorKeyBits));
     unsigned long long hc[4];
     DL_CHECK(cudaGetLastError());
@@ -626,18 +591,18 @@ int build_layout_device(const flbp_graph_desc &g, const DevGraphIn &in, int prec
     }
 
     // --- variable entries and the internal variable order -------------------------------------
-    const uint32_t *vdeg = n_ent_of;
-    uint32_t *first = P.get<uint32_t>(V), *var_of_dev = P.get<uint32_t>(n_slots);
+    uint32_t *vdeg = P.get<uint32_t>(V), *first = P.get<uint32_t>(V), *var_of_dev = P.get<uint32_t>(n_slots);
     uint8_t *is_entry = P.get<uint8_t>(E);
     uint64_t *vkey = P.get<uint64_t>(V), *vkey2 = P.get<uint64_t>(V);
     uint32_t *vidx = P.get<uint32_t>(V), *order = P.get<uint32_t>(V);
     DL_CHECK(P.err);
     DL_CHECK(dalloc_out(&D.int_of_var, (size_t)V, D, st));
+    DL_CHECK(cudaMemsetAsync(vdeg, 0, std::max<int64_t>(1, V) * 4, st));
     DL_CHECK(cudaMemsetAsync(first, 0xff, std::max<int64_t>(1, V) * 4, st));
     DL_CHECK(cudaMemsetAsync(var_of_dev, 0xff, std::max<uint64_t>(1, n_slots) * 4, st));
     DL_CHECK(cudaMemsetAsync(is_entry, 0, std::max<int64_t>(1, E), st));
     if (nf > 0)
-        k_entries<<<grid_for(nf), kTPB, 0, st>>>(in, foi, nf, hstate, dev_slot, is_entry, var_of_dev, first);
+        k_entries<<<grid_for(nf), kTPB, 0, st>>>(in, foi, nf, hstate, dev_slot, is_entry, vdeg, var_of_dev, first);
     DL_CHECK(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long), st));
     if (V > 0) {
         k_var_keys<<<grid_for(V), kTPB, 0, st>>>(vdeg, first, V, vkey, vidx, cnt);

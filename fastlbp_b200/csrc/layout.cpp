@@ -361,108 +361,24 @@ int build_layout(const flbp_graph_desc &g, HostLayout &L, std::string &err, cons
     const uint32_t G = graphs ? graphs->n_graphs : 1;
     auto fgraph = [&](int64_t I) -> uint32_t { return graphs ? graphs->factor_graph[I] : 0u; };
     auto vgraph = [&](int64_t i) -> uint32_t { return graphs ? graphs->var_graph[i] : 0u; };
-    // Links: an AND factor whose head variable has exactly one other entry, a
-    // body slot of an OR factor (a derivation rule's variable), is linked to
-    // that slot. Per variable the number of entries and the exclusive-or of
-    // their (factor, slot) pairs give either end from the other.
-    const bool by_link = G <= 4096;
-    hvec<uint32_t> n_ent_of = par_vec<uint32_t>(by_link ? V : 0, 0);
-    hvec<uint64_t> ends_of = par_vec<uint64_t>(by_link ? V : 0, 0);
-#pragma omp parallel for if (F >= kParMin)
-    for (int64_t I = 0; I < F; I++) {
-        if (!by_link || !active[I]) continue;
-        for (int64_t e = off[I]; e < off[I + 1]; e++) {
-            if (e == g.factor_head[I] && head_state[I] != HEAD_FREE) continue;
-            const size_t v = (size_t)g.slot_var[e];
-            __atomic_fetch_add(&n_ent_of[v], 1u, __ATOMIC_RELAXED);
-            __atomic_fetch_xor(&ends_of[v], (uint64_t)I << 32 | (uint64_t)e, __ATOMIC_RELAXED);
-        }
-    }
-    auto degree = [&](int64_t I) { return (uint64_t)(off[I + 1] - off[I]); };
-    // the linked factor at body slot e of OR factor J, or -1
-    auto linked_at = [&](int64_t J, int64_t e) -> int64_t {
-        const size_t v = (size_t)g.slot_var[e];
-        if (n_ent_of[v] != 2) return -1;
-        const uint64_t o = ends_of[v] ^ ((uint64_t)J << 32 | (uint64_t)e);
-        const int64_t I = (int64_t)(o >> 32), h = (int64_t)(o & 0xffffffffu);
-        const bool ok = I != J && g.factor_type[I] == FLBP_AND && g.factor_head[I] == h &&
-                        degree(I) <= kSellFactorDegree;
-        return ok ? I : -1;
-    };
-    // whether sliced-ELL factor I is linked
-    auto is_linked = [&](int64_t I) -> bool {
-        if (g.factor_type[I] != FLBP_AND || head_state[I] != HEAD_FREE) return false;
-        const int64_t h = g.factor_head[I];
-        const size_t v = (size_t)g.slot_var[h];
-        if (n_ent_of[v] != 2) return false;
-        const uint64_t o = ends_of[v] ^ ((uint64_t)I << 32 | (uint64_t)h);
-        const int64_t J = (int64_t)(o >> 32), e = (int64_t)(o & 0xffffffffu);
-        return J != I && g.factor_type[J] == FLBP_OR && g.factor_head[J] != e;
-    };
     hvec<int64_t> fact_of_int;
     uint32_t nf_sell = 0, nf_big = 0;
     {
-        // Classes (graph, degree) of the sliced-ELL factors, then one class of
-        // the large ones. Within a class the factors that are not linked come
-        // first, in index order; the linked ones follow by the degree class of
-        // their OR factor and then by its slot, so that a group of OR factors
-        // sends its body messages to neighbouring variables and those send
-        // theirs to neighbouring factors.
-        // Measured on the 1M-tuple graph: the factor pass stores to 2.98 M 32-byte
-        // sectors by warp store instead of 3.52 M, the variable pass to 3.05 M
-        // instead of 3.60 M (both passes are bound by that rate, about 167 G
-        // sectors/s). Batches of very many graphs keep the plain order, which
-        // needs no counters per class of OR factor.
+        // classes (graph, degree) of the sliced-ELL factors, then one class of the large ones
         constexpr uint32_t D = kSellFactorDegree + 1;
-        const uint32_t B = by_link ? kSellFactorDegree + 2 : 1;
-        const size_t nk = ((size_t)G * D + 1) * B;
-        auto cls = [&](int64_t I) -> size_t {
-            const uint64_t d = degree(I);
-            return d <= kSellFactorDegree ? (size_t)fgraph(I) * D + d : (size_t)G * D;
-        };
-        auto key = [&](int64_t I) -> size_t {  // factors placed in index order
+        const size_t nk = (size_t)G * D + 1;
+        auto key = [&](int64_t I) -> size_t {
             if (!active[I]) return nk;
-            const size_t c = cls(I);
-            return by_link && c < (size_t)G * D && is_linked(I) ? nk : c * B;
-        };
-        auto lkey = [&](int64_t J, int64_t I) -> size_t {  // those placed by their link
-            return cls(I) * B + std::min<uint64_t>(degree(J), kSellFactorDegree + 1);
-        };
-        auto each_link = [&](int64_t J, auto put) {
-            if (!by_link || !active[J] || g.factor_type[J] != FLBP_OR) return;
-            for (int64_t e = off[J]; e < off[J + 1]; e++) {
-                if (e == g.factor_head[J]) continue;
-                const int64_t I = linked_at(J, e);
-                if (I >= 0) put(I, lkey(J, I));
-            }
+            const uint64_t d = (uint64_t)(off[I + 1] - off[I]);
+            return d <= kSellFactorDegree ? (size_t)fgraph(I) * D + d : nk - 1;
         };
         const Chunks c = chunks(F, nk);
-        std::vector<uint64_t> cnt = class_counts(c, nk, key);
-#pragma omp parallel for schedule(static, 1) if (c.T > 1)
-        for (int t = 0; t < c.T; t++)
-            for (int64_t J = c.lo(t); J < c.hi(t); J++)
-                each_link(J, [&](int64_t, size_t k) { cnt[(size_t)t * nk + k]++; });
+        const std::vector<uint64_t> cnt = class_counts(c, nk, key);
         const std::vector<uint64_t> start = class_starts(c, nk, cnt, 0);
-        nf_sell = (uint32_t)start[(size_t)G * D * B];
-        nf_big = (uint32_t)(start[nk] - start[(size_t)G * D * B]);
+        nf_sell = (uint32_t)start[nk - 1];
+        nf_big = (uint32_t)(start[nk] - start[nk - 1]);
         fact_of_int.resize((size_t)nf_sell + nf_big);  // every position is placed below
-        std::vector<uint64_t> at((size_t)c.T * nk);
-        for (size_t k = 0; k < nk; k++) {
-            uint64_t p = start[k];
-            for (int t = 0; t < c.T; t++) {
-                at[(size_t)t * nk + k] = p;
-                p += cnt[(size_t)t * nk + k];
-            }
-        }
-#pragma omp parallel for schedule(static, 1) if (c.T > 1)
-        for (int t = 0; t < c.T; t++) {
-            uint64_t *a = &at[(size_t)t * nk];
-            for (int64_t I = c.lo(t); I < c.hi(t); I++) {
-                const size_t k = key(I);
-                if (k < nk) fact_of_int[a[k]++] = I;
-                each_link(I, [&](int64_t L_, size_t lk) { fact_of_int[a[lk]++] = L_; });
-            }
-        }
+        class_place(c, nk, cnt, start, key, [&](int64_t I, uint64_t at) { fact_of_int[at] = I; });
         // large factors: those too large for a tile first, then by (graph, decreasing
         // degree); warps deal them round-robin, largest first
         auto deg = [&](int64_t I) { return off[I + 1] - off[I]; };
