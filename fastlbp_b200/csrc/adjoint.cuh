@@ -145,12 +145,13 @@ __device__ __forceinline__ void var_adjoint_reg(const AdjArgs &a, uint32_t iv, u
 // that the narrow groups, the common case, do not pay the registers of the
 // wide ones.
 constexpr uint32_t kNarrowWidth = 8;
+constexpr uint32_t kAdjThreads = 128;  // threads per block of the adjoint kernels
 
-template <typename T, bool WIDE>
-__global__ void var_adjoint_kernel(AdjArgs a, const uint32_t *__restrict__ groups, uint32_t n, const T *__restrict__ fv,
-                                   const T *__restrict__ lam, const T *gS, T *__restrict__ mu,
-                                   T *__restrict__ gprior) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+template <typename T>
+__device__ __forceinline__ void var_adjoint_narrow(const AdjArgs &a, uint32_t block, const uint32_t *__restrict__ groups,
+                                                   uint32_t n, const T *__restrict__ fv, const T *__restrict__ lam,
+                                                   const T *gS, T *__restrict__ mu, T *__restrict__ gprior) {
+    const uint32_t t = block * kAdjThreads + threadIdx.x;
     if ((t >> 5) >= n) return;
     const uint32_t g = groups[t >> 5], iv = 32u * g + (t & 31);
     if (iv >= a.nv_sell) return;
@@ -158,34 +159,26 @@ __global__ void var_adjoint_kernel(AdjArgs a, const uint32_t *__restrict__ group
     const uint32_t w = (a.vg_base[g + 1] - base) >> 5, bl = base + (t & 31);
 #define FLBP_VW(N) \
     case N: var_adjoint_reg<T, N>(a, iv, bl, fv, lam, gS, mu, gprior); break;
-    if (WIDE) {
-        switch (w) {  // warp-uniform
-            FLBP_VW(9) FLBP_VW(10) FLBP_VW(11) FLBP_VW(12) FLBP_VW(13) FLBP_VW(14) FLBP_VW(15) FLBP_VW(16)
-            default: break;
-        }
-    } else {
-        switch (w) {
-            FLBP_VW(1) FLBP_VW(2) FLBP_VW(3) FLBP_VW(4) FLBP_VW(5) FLBP_VW(6) FLBP_VW(7) FLBP_VW(8)
-            default: break;
-        }
+    switch (w) {  // warp-uniform
+        FLBP_VW(1) FLBP_VW(2) FLBP_VW(3) FLBP_VW(4) FLBP_VW(5) FLBP_VW(6) FLBP_VW(7) FLBP_VW(8)
+        default: break;
     }
 #undef FLBP_VW
 }
-static_assert(kSellVarDegree == 16, "var_adjoint_kernel instantiates widths 1..16");
+static_assert(kNarrowWidth == 8, "var_adjoint_narrow instantiates widths 1..8");
 
 // Wide sliced-ELL groups (9-16 entries), two warps per group: warp h of the
 // pair takes entries h, h + 2, ... of the group's 32 variables (one per
 // lane), the pair combines its partial sums in shared memory, and each warp
 // writes the mu of its own entries. Blocks of 128 threads hold two groups.
 template <typename T>
-__global__ void __launch_bounds__(128) var_adjoint_wide_kernel(AdjArgs a, const uint32_t *__restrict__ groups,
-                                                                uint32_t n, const T *__restrict__ fv,
-                                                                const T *__restrict__ lam, const T *gS,
-                                                                T *__restrict__ mu, T *__restrict__ gprior) {
+__device__ __forceinline__ void var_adjoint_wide(const AdjArgs &a, uint32_t block, const uint32_t *__restrict__ groups,
+                                                 uint32_t n, const T *__restrict__ fv, const T *__restrict__ lam,
+                                                 const T *gS, T *__restrict__ mu, T *__restrict__ gprior) {
     __shared__ int s_cnt[4][32][2];
     __shared__ T s_sum[4][32][3];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = warp & 1;
-    const uint32_t gi = 2 * blockIdx.x + (warp >> 1);
+    const uint32_t gi = 2 * block + (warp >> 1);
     const bool live_g = gi < n;
     const uint32_t g = live_g ? groups[gi] : 0u, iv = 32u * g + lane;
     const bool live = live_g && iv < a.nv_sell;
@@ -250,9 +243,10 @@ __global__ void __launch_bounds__(128) var_adjoint_wide_kernel(AdjArgs a, const 
 constexpr int kBigVarLanes = 8, kBigVarRegs = 8;
 
 template <typename T>
-__global__ void var_adjoint_big_kernel(AdjArgs a, const T *__restrict__ fv, const T *__restrict__ lam, const T *gS,
-                                       T *__restrict__ mu, T *__restrict__ gprior) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void var_adjoint_big(const AdjArgs &a, uint32_t block, const T *__restrict__ fv,
+                                                const T *__restrict__ lam, const T *gS, T *__restrict__ mu,
+                                                T *__restrict__ gprior) {
+    const uint32_t t = block * kAdjThreads + threadIdx.x;
     const uint32_t b = t / kBigVarLanes, j = t % kBigVarLanes;
     // whole warps stay in the shuffles below; lanes past the last variable carry no entries
     const bool live = b < a.nv_big;
@@ -309,6 +303,25 @@ __global__ void var_adjoint_big_kernel(AdjArgs a, const T *__restrict__ fv, cons
     for (int r = 0; r < kBigVarRegs; r++) put(sr[r], xr[r], lr[r]);
     for (uint32_t e = e0 + j + kBigVarRegs * kBigVarLanes; e < e1; e += kBigVarLanes) put(a.v_ent[e], fv[e], lam[e]);
     if (j == 0 && folded) gprior[iv] += Lam + gs;
+}
+
+// The variable adjoint of a step in one launch: blocks [0, wide) the wide
+// groups, the next `big` blocks the large variables, the rest the narrow
+// groups. At a few hundred thousand slots each part alone is a launch of
+// mostly latency: three launches took 7.1 + 6.6 + 5.7 us a step on two graphs
+// of 50 k tuples (cold, one B200).
+template <typename T>
+__global__ void __launch_bounds__(kAdjThreads) var_adjoint_kernel(AdjArgs a, const uint32_t *__restrict__ narrow_groups,
+                                                                  uint32_t n_narrow,
+                                                                  const uint32_t *__restrict__ wide_groups,
+                                                                  uint32_t n_wide, uint32_t wide_blocks,
+                                                                  uint32_t big_blocks, const T *__restrict__ fv,
+                                                                  const T *__restrict__ lam, const T *gS,
+                                                                  T *__restrict__ mu, T *__restrict__ gprior) {
+    const uint32_t b = blockIdx.x;
+    if (b < wide_blocks) var_adjoint_wide<T>(a, b, wide_groups, n_wide, fv, lam, gS, mu, gprior);
+    else if (b < wide_blocks + big_blocks) var_adjoint_big<T>(a, b - wide_blocks, fv, lam, gS, mu, gprior);
+    else var_adjoint_narrow<T>(a, b - wide_blocks - big_blocks, narrow_groups, n_narrow, fv, lam, gS, mu, gprior);
 }
 
 // Factor adjoint of one sliced-ELL factor (group width W, one lane): slot k
@@ -394,10 +407,10 @@ __device__ __forceinline__ void factor_adjoint_reg(const AdjArgs &a, uint32_t ba
 }
 
 template <typename T, bool WIDE>
-__global__ void __launch_bounds__(128, (!WIDE && sizeof(T) == 4) ? 8 : 1) factor_adjoint_sell_kernel(AdjArgs a, const uint32_t *__restrict__ groups, uint32_t n,
-                                           const T *__restrict__ vf, const T *__restrict__ mu, T *__restrict__ lam,
-                                           T *__restrict__ gp, T *__restrict__ gq) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void factor_adjoint_sell(const AdjArgs &a, uint32_t block, const uint32_t *__restrict__ groups,
+                                                    uint32_t n, const T *__restrict__ vf, const T *__restrict__ mu,
+                                                    T *__restrict__ lam, T *__restrict__ gp, T *__restrict__ gq) {
+    const uint32_t t = block * kAdjThreads + threadIdx.x;
     if ((t >> 5) >= n) return;
     const uint32_t g = groups[t >> 5], f = 32u * g + (t & 31);
     if (f >= a.nf_sell) return;
@@ -422,15 +435,16 @@ __global__ void __launch_bounds__(128, (!WIDE && sizeof(T) == 4) ? 8 : 1) factor
     }
 #undef FLBP_FW
 }
-static_assert(kSellFactorDegree == 16, "factor_adjoint_sell_kernel instantiates widths 2..16");
+static_assert(kSellFactorDegree == 16, "factor_adjoint_sell instantiates widths 2..16");
 
 // Big factors, one warp each: leave-one-out products from a sum of
 // log-sigmoids with a count of exact zeros (inputs at -inf after the
 // orientation sign).
 template <typename T>
-__global__ void factor_adjoint_big_kernel(AdjArgs a, const T *__restrict__ vf, const T *__restrict__ mu,
-                                          T *__restrict__ lam, T *__restrict__ gp, T *__restrict__ gq) {
-    const uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+__device__ __forceinline__ void factor_adjoint_big(const AdjArgs &a, uint32_t block, const T *__restrict__ vf,
+                                                   const T *__restrict__ mu, T *__restrict__ lam, T *__restrict__ gp,
+                                                   T *__restrict__ gq) {
+    const uint32_t b = (block * kAdjThreads + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (b >= a.nf_big) return;
     const uint32_t f = a.nf_sell + b, s0 = a.fb_off[b], s1 = s0 + a.fb_deg[b];
@@ -510,6 +524,18 @@ __global__ void factor_adjoint_big_kernel(AdjArgs a, const T *__restrict__ vf, c
         gp[f] += dgp;
         if (gq) gq[f] += dgq;
     }
+}
+
+// The factor adjoint of a step: blocks [0, big) the large factors, the rest
+// the sliced-ELL groups of one width class (wide groups in a launch of their
+// own, for their registers).
+template <typename T, bool WIDE>
+__global__ void __launch_bounds__(kAdjThreads, (!WIDE && sizeof(T) == 4) ? 8 : 1)
+    factor_adjoint_kernel(AdjArgs a, const uint32_t *__restrict__ groups, uint32_t n, uint32_t big_blocks,
+                          const T *__restrict__ vf, const T *__restrict__ mu, T *__restrict__ lam, T *__restrict__ gp,
+                          T *__restrict__ gq) {
+    if (blockIdx.x < big_blocks) factor_adjoint_big<T>(a, blockIdx.x, vf, mu, lam, gp, gq);
+    else factor_adjoint_sell<T, WIDE>(a, blockIdx.x - big_blocks, groups, n, vf, mu, lam, gp, gq);
 }
 
 // dL/dS_v = dL/db_v * b_v (1 - b_v) at the final beliefs, from the loss

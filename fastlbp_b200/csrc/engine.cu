@@ -853,7 +853,7 @@ bool use_resident(flbp_engine *e, int mode) {
 }
 
 template <typename T>
-cudaError_t launch_resident_t(flbp_engine *e, int mode, uint32_t cap, bool final_beliefs) {
+ResArgs<T> resident_args(flbp_engine *e, int mode, uint32_t cap, bool final_beliefs) {
     ResArgs<T> r;
     r.f = factor_args<T>(e);
     r.v = var_args(e);
@@ -873,7 +873,13 @@ cudaError_t launch_resident_t(flbp_engine *e, int mode, uint32_t cap, bool final
     r.final_beliefs = final_beliefs ? 1 : 0;
     r.rows_f = e->res_rows_f;
     r.rows_v = e->res_rows_v;
-    return resident_launch<T>(e->damping != 0.0, e->res_plan == 2, e->res_grid, e->res_smem, r, e->stream);
+    return r;
+}
+
+template <typename T>
+cudaError_t launch_resident_t(flbp_engine *e, int mode, uint32_t cap, bool final_beliefs) {
+    return resident_launch<T>(e->damping != 0.0, e->res_plan == 2, e->res_grid, e->res_smem,
+                              resident_args<T>(e, mode, cap, final_beliefs), e->stream);
 }
 
 
@@ -2814,25 +2820,25 @@ void launch_adjoint_step(flbp_engine *e, const void *vf, const void *fv, const v
     const uint32_t *c = e->adj_group_n;  // narrow var, wide var, narrow factor, wide factor groups
     const uint32_t o1 = c[0], o2 = o1 + c[1], o3 = o2 + c[2];
     int n = 0;
-    auto go = [&](uint32_t cnt) { n += cnt ? 1 : 0; return cnt != 0; };
-    if (go(c[0]))
-        var_adjoint_kernel<T, false><<<blocks_for(32ull * c[0], 128), 128, 0, e->stream>>>(
-            a, gl, c[0], (const T *)fv, (const T *)lam_next, (const T *)gs, mu, gprior);
-    if (go(c[1]))
-        var_adjoint_wide_kernel<T><<<(unsigned)((c[1] + 1) / 2), 128, 0, e->stream>>>(
-            a, gl + o1, c[1], (const T *)fv, (const T *)lam_next, (const T *)gs, mu, gprior);
-    if (go(a.nv_big))
-        var_adjoint_big_kernel<T><<<blocks_for((uint64_t)kBigVarLanes * a.nv_big, 128), 128, 0, e->stream>>>(
-            a, (const T *)fv, (const T *)lam_next, (const T *)gs, mu, gprior);
-    if (go(c[2]))
-        factor_adjoint_sell_kernel<T, false><<<blocks_for(32ull * c[2], 128), 128, 0, e->stream>>>(
-            a, gl + o2, c[2], (const T *)vf, mu, (T *)lam, gp, gq);
-    if (go(c[3]))
-        factor_adjoint_sell_kernel<T, true><<<blocks_for(32ull * c[3], 128), 128, 0, e->stream>>>(
-            a, gl + o3, c[3], (const T *)vf, mu, (T *)lam, gp, gq);
-    if (go(a.nf_big))
-        factor_adjoint_big_kernel<T><<<blocks_for(32ull * a.nf_big, 128), 128, 0, e->stream>>>(a, (const T *)vf, mu,
-                                                                                                (T *)lam, gp, gq);
+    const unsigned wide_b = (c[1] + 1) / 2, big_vb = a.nv_big ? blocks_for((uint64_t)kBigVarLanes * a.nv_big, kAdjThreads) : 0;
+    const unsigned narrow_vb = c[0] ? blocks_for(32ull * c[0], kAdjThreads) : 0;
+    if (wide_b + big_vb + narrow_vb) {
+        n++;
+        var_adjoint_kernel<T><<<wide_b + big_vb + narrow_vb, kAdjThreads, 0, e->stream>>>(
+            a, gl, c[0], gl + o1, c[1], wide_b, big_vb, (const T *)fv, (const T *)lam_next, (const T *)gs, mu, gprior);
+    }
+    const unsigned big_fb = a.nf_big ? blocks_for(32ull * a.nf_big, kAdjThreads) : 0;
+    const unsigned narrow_fb = c[2] ? blocks_for(32ull * c[2], kAdjThreads) : 0;
+    if (big_fb + narrow_fb) {
+        n++;
+        factor_adjoint_kernel<T, false><<<big_fb + narrow_fb, kAdjThreads, 0, e->stream>>>(
+            a, gl + o2, c[2], big_fb, (const T *)vf, mu, (T *)lam, gp, gq);
+    }
+    if (c[3]) {
+        n++;
+        factor_adjoint_kernel<T, true><<<blocks_for(32ull * c[3], kAdjThreads), kAdjThreads, 0, e->stream>>>(
+            a, gl + o3, c[3], 0u, (const T *)vf, mu, (T *)lam, gp, gq);
+    }
     e->launches += n;
 }
 
@@ -2875,6 +2881,39 @@ char *adj_seg_fv(flbp_engine *e, long long i) {
 // checkpoint, and the last segment keeps every state in the segment buffers
 // (its final variable pass writes the engine's vf, and fv_{T-1} is copied
 // to the engine's fv, so the engine state is that of T plain sweeps).
+// n sweeps of a segment from v0: f->v messages of sweep i to fseg + i
+// fstride, v->f messages to vseg + (i + 1) vstride (elements), the last ones
+// to vlast (null: none). One launch of the resident kernel where the graph
+// is of its size, else two launches a sweep.
+template <typename T>
+int adjoint_sweeps(flbp_engine *e, long long n, const T *v0, T *vseg, size_t vstride, T *fseg, size_t fstride,
+                   T *vlast) {
+    if (use_resident(e, 1)) {  // up to the larger limit: without it every sweep is two launches that no graph replays
+        for (long long i = 0; i < n; i += kResSweeps) {
+            const long long m = std::min<long long>(kResSweeps, n - i);
+            ResArgs<T> r = resident_args<T>(e, 0, (uint32_t)m, false);
+            r.states = 1;
+            r.v0 = i == 0 ? v0 : vseg + (size_t)i * vstride;
+            r.vseg = vseg + (size_t)i * vstride;
+            r.fseg = fseg + (size_t)i * fstride;
+            r.vstride = vstride;
+            r.fstride = fstride;
+            r.vlast = i + m < n ? r.vseg + (size_t)m * vstride : vlast;
+            FLBP_CUDA(cudaMemsetAsync(reinterpret_cast<char *>(e->d_ctl) + offsetof(Ctl, rs), 0, sizeof(ResSync),
+                                      e->stream));
+            FLBP_CUDA(resident_launch<T>(false, e->res_plan == 2, e->res_grid, e->res_smem, r, e->stream));
+            e->launches += 1;
+        }
+        return FLBP_OK;
+    }
+    for (long long i = 0; i < n; i++) {
+        T *vout = i + 1 < n ? vseg + (size_t)(i + 1) * vstride : vlast;
+        launch_factor_pass_on<T>(e, i == 0 ? v0 : vseg + (size_t)i * vstride, fseg + (size_t)i * fstride);
+        if (vout) launch_var_pass_on<T>(e, fseg + (size_t)i * fstride, vout);
+    }
+    return FLBP_OK;
+}
+
 template <typename T>
 int adjoint_forward_t(flbp_engine *e, long long T_, long long K) {
     const size_t ns = std::max<uint64_t>(1, e->L.n_slots);
@@ -2884,13 +2923,12 @@ int adjoint_forward_t(flbp_engine *e, long long T_, long long K) {
     for (long long c = 0; c < nck; c++) {
         const long long n1 = std::min<long long>(K, T_ - c * K);
         const bool last = c == nck - 1;
-        for (long long i = 0; i < n1; i++) {
-            const void *vin = i == 0 ? adj_ckpt(e, c) : (last ? adj_seg_vf(e, c, i) : e->d_vf);
-            void *fout = last ? adj_seg_fv(e, i) : e->d_fv;
-            void *vout = i + 1 < n1 ? (last ? adj_seg_vf(e, c, i + 1) : e->d_vf) : (last ? e->d_vf : adj_ckpt(e, c + 1));
-            launch_factor_pass_on<T>(e, vin, fout);
-            launch_var_pass_on<T>(e, fout, vout);
-        }
+        const size_t ne = std::max<size_t>(1, e->n_ent);
+        // sweep i of the last segment reads state i of the segment buffers, those before it the engine's own arrays
+        if (int rc = adjoint_sweeps<T>(e, n1, (const T *)adj_ckpt(e, c), last ? (T *)e->d_seg_vf : (T *)e->d_vf,
+                                       last ? ns : 0, last ? (T *)e->d_seg_fv : (T *)e->d_fv, last ? ne : 0,
+                                       last ? (T *)e->d_vf : (T *)adj_ckpt(e, c + 1)))
+            return rc;
         if (last && e->n_ent)
             FLBP_CUDA(cudaMemcpyAsync(e->d_fv, adj_seg_fv(e, n1 - 1), e->n_ent * e->tsize, cudaMemcpyDeviceToDevice,
                                       e->stream));
@@ -2993,10 +3031,9 @@ int adjoint_backward_t(flbp_engine *e, const double *grad_b, double *gp_out, dou
         // the segment's states: vf_i = adj_seg_vf(c, i), fv_i in seg_fv(i), recomputed
         // from the checkpoint unless the forward run left them (last segment)
         if (!(c == nck - 1 && e->adj_last_seg)) {
-            for (long long i = 0; i < n1; i++) {
-                launch_factor_pass_on<T>(e, adj_seg_vf(e, c, i), adj_seg_fv(e, i));
-                if (i + 1 < n1) launch_var_pass_on<T>(e, adj_seg_fv(e, i), adj_seg_vf(e, c, i + 1));
-            }
+            if ((rc = adjoint_sweeps<T>(e, n1, (const T *)adj_ckpt(e, c), (T *)e->d_seg_vf, ns, (T *)e->d_seg_fv, ne,
+                                        nullptr)))
+                return rc;
         }
         e->adj_last_seg = false;  // the segment buffers are reused from here on
         for (long long i = n1 - 1; i >= 0; i--) {

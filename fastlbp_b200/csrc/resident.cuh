@@ -50,6 +50,14 @@ struct ResArgs {
     uint32_t cap;          // sweeps of this launch at most
     int final_beliefs;     // fixed runs: the last sweep also writes the beliefs
     uint32_t rows_f, rows_v;  // items per block of each pass (the last row may be short)
+    // Runs that keep states (gradients): sweep s reads v0 (s = 0) or vseg +
+    // s vstride, writes its f->v messages to fseg + s fstride and its v->f
+    // messages to vseg + (s + 1) vstride, the last sweep to vlast, or, when
+    // that is null, no v->f messages. Without states all sweeps use vf and fv.
+    int states = 0;
+    const T *v0 = nullptr;
+    T *vseg = nullptr, *fseg = nullptr, *vlast = nullptr;
+    uint64_t vstride = 0, fstride = 0;
 };
 
 // Shared-memory words of one cached item: positions of its W columns (a large
@@ -312,8 +320,8 @@ __global__ void __launch_bounds__(kResThreads, sizeof(T) == 4 ? 2 : 1) resident_
             for (uint32_t w = tid; w < gwords; w += kResThreads) rs->moved[nslot][w] = 0u;
         }
         for (uint32_t w = tid; w < gwords; w += kResThreads) s_moved[w] = 0u;
-        const T *vf = r.vf;
-        T *fv = r.fv;
+        const T *vf = !r.states ? r.vf : s == 0 ? r.v0 : r.vseg + s * r.vstride;
+        T *fv = !r.states ? r.fv : r.fseg + s * r.fstride;
         for (uint32_t h = b; h < r.f.nf_huge; h += nb) {
             if (batch && stopped(r.f.f_graph[r.f.nf_sell + h])) continue;
             factor_block_huge<T>(r.f, h, tid, CgPtr<T>{vf}, fv, s_l, s_a);
@@ -359,6 +367,12 @@ __global__ void __launch_bounds__(kResThreads, sizeof(T) == 4 ? 2 : 1) resident_
                                              lane, fv);
             }
         }
+        const bool last = s + 1 == r.cap;
+        T *vout = !r.states ? r.vf : last ? r.vlast : r.vseg + (s + 1) * r.vstride;
+        if (!vout) {  // the last sweep's f->v messages end the run
+            s++;
+            break;
+        }
         target += nb;
         __syncthreads();
         if (tid == 0 && !res_arrive_wait(&rs->arrive, target)) s_stop = 2;
@@ -366,7 +380,6 @@ __global__ void __launch_bounds__(kResThreads, sizeof(T) == 4 ? 2 : 1) resident_
         if (s_stop) break;
 
         // ---- variable phase
-        const bool last = s + 1 == r.cap;
         const int bm = mode == 3 ? 1 : mode != 0 ? mode : (last && r.final_beliefs) ? 3 : 0;
         const double pscale = s_pscale;
         double dmax = 0.0;
@@ -376,7 +389,7 @@ __global__ void __launch_bounds__(kResThreads, sizeof(T) == 4 ? 2 : 1) resident_
             if (batch && stopped(g)) continue;
             double dd = 0.0;
 #define FLBP_HUGE(M) \
-    var_block_huge<T, M, true, DAMP, true>(va, h, tid, r.fv, r.vf, r.fvd, r.d, pscale, tol, cnt, s_l, s_a, s_b)
+    var_block_huge<T, M, true, DAMP, true>(va, h, tid, fv, vout, r.fvd, r.d, pscale, tol, cnt, s_l, s_a, s_b)
             if (bm == 0) dd = FLBP_HUGE(0);
             else if (bm == 1) dd = FLBP_HUGE(1);
             else if (bm == 2) dd = FLBP_HUGE(2);
@@ -388,8 +401,7 @@ __global__ void __launch_bounds__(kResThreads, sizeof(T) == 4 ? 2 : 1) resident_
         for (uint32_t j = wid; j < r.rows_v; j += kConsumerWarps) {
             const uint32_t it = res_item_of(j, b, nb);
             if (it >= n_v) break;
-            const T *fv = r.fv;
-            T *vf = r.vf, *fvd = r.fvd;
+            T *fvd = r.fvd;
             const ResRow x = CACHE ? rows[r.rows_f + j] : v_row(it);
             const uint32_t *ent = CACHE ? sm + x.off : va.v_ent + x.base;
             const bool big = it < nvb;
@@ -416,17 +428,17 @@ __global__ void __launch_bounds__(kResThreads, sizeof(T) == 4 ? 2 : 1) resident_
                 auto old = [&](uint32_t k) { return DAMP ? fvd[k0 + k] : T(0); };
                 var_warp_sum<T, DAMP>(in, old, x.w, prior, pidx, r.d, pscale, lane, S, npos, nneg);
                 var_warp_send<T, DAMP, true>(in, old, [&](uint32_t k) { return ent[k]; }, DAMP ? fvd + k0 : nullptr,
-                                             x.w, r.d, lane, S, npos, nneg, GlobalOut<T>{vf});
+                                             x.w, r.d, lane, S, npos, nneg, GlobalOut<T>{vout});
                 Sv = AccOps<typename WideAcc<T>::type>::value(S);
             } else {
                 typedef typename NarrowAcc<T>::type A;
                 A S = AccOps<A>::zero();
                 if (real) decode_prior<T>(prior, pidx, pscale, S, npos, nneg);
                 if (x.w <= (uint32_t)kResNarrow)
-                    res_var_group<T, kResNarrow, DAMP, CACHE>(x.w, fv, vf, fvd, r.d, x.base, live, ent, lane, S,
+                    res_var_group<T, kResNarrow, DAMP, CACHE>(x.w, fv, vout, fvd, r.d, x.base, live, ent, lane, S,
                                                               npos, nneg);
                 else
-                    res_var_group<T, kSellVarDegree, DAMP, CACHE>(x.w, fv, vf, fvd, r.d, x.base, live, ent, lane,
+                    res_var_group<T, kSellVarDegree, DAMP, CACHE>(x.w, fv, vout, fvd, r.d, x.base, live, ent, lane,
                                                                   S, npos, nneg);
                 Sv = AccOps<A>::value(S);
             }
