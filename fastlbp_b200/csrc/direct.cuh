@@ -124,7 +124,11 @@ template <typename T, int MINB, bool SETS = false>
 __global__ void __launch_bounds__(kDirectThreads, MINB) factor_direct_kernel(FactorArgs a, const T *__restrict__ vf,
                                                                              T *__restrict__ fv, Ctl *ctl) {
     if (*(volatile int *)&ctl->done) return;
-    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) sweep_open(ctl);
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
+        unsigned long long now;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+        sweep_open(ctl, now);
+    }
     if (SETS) {
         if (a.set_done[blockIdx.y]) return;
         vf += blockIdx.y * a.set_vf_stride;

@@ -96,8 +96,9 @@ struct flbp_engine {
     void *d_lam = nullptr, *d_lam2 = nullptr, *d_mu = nullptr, *d_gp = nullptr, *d_gq = nullptr;
     void *d_gprior = nullptr, *d_gs = nullptr;
     size_t adj_ckpt_n = 0, adj_seg_n = 0;
-    // staged factor pass: each block's tiles (FactorArgs::tile_list / tile_off)
-    uint32_t *d_ftlist = nullptr, *d_ftoff = nullptr;
+    // staged factor pass: the headers of each block's tiles (FactorArgs::dealt)
+    uint32_t *d_ftdealt = nullptr;
+    uint32_t ft_per_block = 0;
     uint32_t *d_int_of_var = nullptr, *d_f_of_int = nullptr;  // caller variable -> internal; internal factor -> caller
     uint32_t *d_pri_fac = nullptr, *d_pri_var = nullptr;      // folded constants: caller factor, internal variable
     double *d_pri_coef = nullptr;                             // their d(constant)/dp
@@ -234,8 +235,8 @@ FactorArgs factor_args(flbp_engine *e) {
     a.nf_huge = e->L.nf_huge;
     a.n_fgroups = e->L.n_fgroups();
     a.thdr = reinterpret_cast<const uint4 *>(e->d_ftiles);
-    a.tile_list = e->d_ftlist;
-    a.tile_off = e->d_ftoff;
+    a.dealt = reinterpret_cast<const uint4 *>(e->d_ftdealt);
+    a.per_block = e->ft_per_block;
     a.n_tiles = e->L.n_ftiles;
     a.n_tile_blocks = e->f_tile_blocks;
     a.f_graph = nullptr;
@@ -1507,6 +1508,15 @@ void adopt_dev_layout(flbp_engine *e, DevLayout &D) {
     D = DevLayout();
 }
 
+// Tile headers in the order of a list (kSentinel: none, an empty header).
+__global__ void dealt_headers_kernel(const uint4 *__restrict__ hdr, const uint32_t *__restrict__ tile, uint32_t n,
+                                     uint4 *__restrict__ out) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, w = kHdrWords / 4;
+    if (i >= n * w) return;
+    const uint32_t t = tile[i / w];
+    out[i] = t == kSentinel ? make_uint4(0u, 0u, 0u, 0u) : hdr[(size_t)t * w + i % w];
+}
+
 // Deals the tiles of a pass to its `nb` blocks so that every block's total
 // cost is about the same (largest first, each to the least loaded block;
 // the huge items a block takes first count towards its load). A tile costs
@@ -1845,9 +1855,24 @@ int create_engine(const flbp_graph_desc *graph, const flbp_engine_opts *opts, fl
         for (uint32_t b = 0; b < L.nf_huge; b++) fh[b % e->factor_grid] += (double)L.fb_deg[b];
         std::vector<uint32_t> fl, fo;
         deal_tiles(L.fhdr, L.n_ftiles, (uint32_t)e->factor_grid, kTileCostFactorItem, fh, fl, fo);
-        if ((rc = dalloc(e, &e->d_ftlist, fl.size())) || (rc = upload(e, e->d_ftlist, fl)) ||
-            (rc = dalloc(e, &e->d_ftoff, fo.size())) || (rc = upload(e, e->d_ftoff, fo)))
+        uint32_t per = 1;
+        for (int b = 0; b < e->factor_grid; b++) per = std::max(per, fo[b + 1] - fo[b]);
+        std::vector<uint32_t> tile((size_t)per * e->factor_grid, kSentinel);
+        for (int b = 0; b < e->factor_grid; b++)
+            std::copy(fl.begin() + fo[b], fl.begin() + fo[b + 1], tile.begin() + (size_t)b * per);
+        uint32_t *d_tile = nullptr;
+        if ((rc = dalloc(e, &e->d_ftdealt, tile.size() * kHdrWords)) || (rc = dalloc(e, &d_tile, tile.size())) ||
+            (rc = upload(e, d_tile, tile))) {
+            if (d_tile) dfree(e, d_tile);
             return fail(rc);
+        }
+        const uint32_t n = (uint32_t)tile.size();
+        dealt_headers_kernel<<<(n * (kHdrWords / 4) + 255) / 256, 256, 0, e->stream>>>(
+            reinterpret_cast<const uint4 *>(e->d_ftiles), d_tile, n, reinterpret_cast<uint4 *>(e->d_ftdealt));
+        e->ft_per_block = per;
+        dfree(e, d_tile);
+        e->bytes -= tile.size() * sizeof(uint32_t);
+        FLBP_CUDA(cudaGetLastError());
         FLBP_CUDA(cudaStreamSynchronize(e->stream));
     }
     e->create_us[3] = us(t_begin, clk()) - e->create_us[0] - e->create_us[1] - e->create_us[2];
@@ -1980,7 +2005,7 @@ int flbp_engine_destroy(flbp_engine *e) {
     if (e->d_set_cut) cudaFree(e->d_set_cut);
     for (void *b : {(void *)e->d_cl_jobs, (void *)e->d_cl_map, (void *)e->d_gdiff, (void *)e->d_cut_ent})
         if (b) cudaFree(b);
-    for (void *b : {(void *)e->d_ftlist, (void *)e->d_ftoff, (void *)e->d_act_f, (void *)e->d_act_v,
+    for (void *b : {(void *)e->d_ftdealt, (void *)e->d_act_f, (void *)e->d_act_v,
                     (void *)e->d_act_flag, e->d_cub_tmp})
         if (b) cudaFree(b);
     for (void *b : {(void *)e->d_fbt_src, (void *)e->d_vbt_src, (void *)e->d_pri_uvar, (void *)e->d_pri_uoff,

@@ -246,9 +246,11 @@ struct FactorArgs {
     const uint2 *trange;      // batched solves: per tile, the range of its items' graphs
     uint32_t n_graphs;        // batched solves: number of graphs
     uint32_t nf_sell, nf_big, nf_huge, n_fgroups, n_tiles, n_tile_blocks;
-    // Staged form on one graph: block b's tiles tile_list[tile_off[b] ..
-    // tile_off[b + 1]) (null: tiles b, b + gridDim.x, ...).
-    const uint32_t *tile_list = nullptr, *tile_off = nullptr;
+    // Staged form on one graph: headers of block b's tiles at dealt + (b
+    // per_block + i) kHdrWords words, i < per_block, those past its last tile
+    // with 0 items (null: tiles b, b + gridDim.x, ...).
+    const uint4 *dealt = nullptr;
+    uint32_t per_block = 0;
     // Staged form of a batched solve: the tiles that hold a live graph,
     // act_list[0 .. *n_act) (null: every tile).
     const uint32_t *act_list = nullptr;
@@ -510,23 +512,27 @@ __device__ __forceinline__ bool graph_done(const uint32_t *s_done, const int *gd
 }
 
 // Producer warp of a pass. A single graph's pass walks the block's own
-// tiles in order: the list the engine dealt it (tile_list / tile_off, tiles
-// of about equal total cost per block, so that all SMs finish together), or
-// without a list tiles blockIdx.x + i gridDim.x. A batched solve instead takes chunks of kChunkTiles consecutive
+// tiles in order: the ones the engine dealt it (dealt / per_block, tiles of
+// about equal total cost per block, so that all SMs finish together; their
+// headers lie together, so that the first copies wait for one load and not
+// for a list and its bounds as well), or without them tiles blockIdx.x + i
+// gridDim.x. A batched solve instead takes chunks of kChunkTiles consecutive
 // tiles from the pass's counter, so that blocks whose tiles belong to stopped
 // graphs take more, and leaves out tiles whose graphs have all stopped. One
 // stage per remaining tile is filled with fill(stage, header in shared
 // memory, full barrier); a stage whose header word 1 is kEndTile closes the
-// stream. All lanes call it; lane 0 issues the copies. After a timeout it
-// records FLBP_ERR_TIMEOUT, lets its own copies land and returns false.
+// stream. `done` (a stopped run) is looked at only after the first headers
+// have been asked for. All lanes call it; lane 0 issues the copies. After a
+// timeout it records FLBP_ERR_TIMEOUT, lets its own copies land and returns
+// false.
 constexpr uint32_t kChunkTiles = 4;
 
 template <int STAGES, typename Fill>
-__device__ bool produce_tiles(const uint4 *thdr, const uint2 *trange, const uint32_t *tile_list,
-                              const uint32_t *tile_off, const uint32_t *act_list, const unsigned int *n_act,
-                              const uint32_t *s_done, const int *gdone, uint32_t n_tiles, unsigned int *counter,
-                              unsigned char *smem, size_t stage_bytes, uint64_t *full, uint64_t *empty, int lane,
-                              Ctl *ctl, Fill fill) {
+__device__ bool produce_tiles(const uint4 *thdr, const uint2 *trange, const uint4 *dealt, uint32_t per_block,
+                              const uint32_t *act_list, const unsigned int *n_act, const uint32_t *s_done,
+                              const int *gdone, uint32_t n_tiles, unsigned int *counter, unsigned char *smem,
+                              size_t stage_bytes, uint64_t *full, uint64_t *empty, int lane, Ctl *ctl, int done,
+                              Fill fill) {
     uint32_t issued = 0;
     bool ok = true;
     const bool dynamic = trange != nullptr;
@@ -534,15 +540,11 @@ __device__ bool produce_tiles(const uint4 *thdr, const uint2 *trange, const uint
     const uint32_t width = dynamic ? kChunkTiles : 32u;
     const uint32_t nb = gridDim.x;
     uint32_t round = dynamic ? __shfl_sync(0xffffffffu, lane == 0 ? atomicAdd(counter, 1u) : 0u, 0) : 0u;
-    const bool listed = !dynamic && tile_list != nullptr;
-    const uint32_t l0 = listed ? tile_off[blockIdx.x] : 0u, ln = listed ? tile_off[blockIdx.x + 1] - l0 : 0u;
+    const bool listed = !dynamic && dealt != nullptr;
     const bool live_list = dynamic && act_list != nullptr;
     const uint32_t n_live = live_list ? *(volatile const unsigned int *)n_act : 0u;
     auto tile_at = [&](uint32_t r, uint32_t k) -> uint32_t {  // n_tiles when out of range
-        if (listed) {
-            const uint64_t i = (uint64_t)r * width + k;
-            return i < ln ? tile_list[l0 + i] : n_tiles;
-        }
+        if (listed) return (uint64_t)r * width + k < per_block ? 0u : n_tiles;  // the header says which tile, if any
         if (live_list) {
             const uint64_t i = (uint64_t)r * width + k;
             return i < n_live ? act_list[i] : n_tiles;
@@ -567,7 +569,9 @@ __device__ bool produce_tiles(const uint4 *thdr, const uint2 *trange, const uint
         }
         uint32_t bits = __ballot_sync(0xffffffffu, act);
         if (act) {  // global -> shared without registers (16 B asynchronous copies)
-            const uint4 *src = thdr + (size_t)(kHdrWords / 4) * t;
+            const uint4 *src = listed ? dealt + (size_t)(kHdrWords / 4) * ((size_t)blockIdx.x * per_block +
+                                                                           (size_t)round * width + lane)
+                                      : thdr + (size_t)(kHdrWords / 4) * t;
             const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&s_hdr[lane][0]);
 #pragma unroll
             for (int i = 0; i < kHdrWords / 4; i++)
@@ -575,6 +579,8 @@ __device__ bool produce_tiles(const uint4 *thdr, const uint2 *trange, const uint
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
         __syncwarp();
+        if (done) return true;  // nothing of this block is in flight
+        if (listed) bits = __ballot_sync(0xffffffffu, act && reinterpret_cast<const uint32_t *>(&s_hdr[lane][0])[1] != 0u);
         if (lane == 0) {
             int j = bits ? __ffs(bits) - 1 : -1;
             while (j >= 0) {
@@ -1002,11 +1008,10 @@ __device__ __forceinline__ void factor_tile_item(VB vb, const uint32_t *ps, uint
 }
 static_assert(kBigFactorBody == 256, "factor_tile_item covers bodies of up to 256 slots");
 
-// Opens a sweep (thread 0 of block 0 of the factor pass, either form): sweep
-// counters, damping weight of the constant priors, residual reset.
-__device__ __forceinline__ void sweep_open(Ctl *ctl) {
-    unsigned long long now;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+// Opens a sweep (one thread of block 0 of the factor pass, either form): sweep
+// counters, damping weight of the constant priors, residual reset. Nothing of
+// it is read before the variable pass. now: %globaltimer at the pass's start.
+__device__ __forceinline__ void sweep_open(Ctl *ctl, unsigned long long now) {
     if (ctl->run_sweeps == 0) ctl->t_start_ns = now;
     ctl->t += 1;
     ctl->run_sweeps += 1;
@@ -1033,8 +1038,9 @@ __global__ void __launch_bounds__(kBlockThreadsDev) factor_pass_kernel(FactorArg
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) uint64_t full[STAGES], empty[STAGES];
     typedef FactorStage<T, GID> FS;
-    if (*(volatile int *)&ctl->done) return;
-    if (blockIdx.x == 0 && threadIdx.x == 0) sweep_open(ctl);
+    const int done = *(volatile int *)&ctl->done;  // looked at once the first loads are on their way
+    unsigned long long opened = 0;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(opened));
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t n_tiles = a.n_tiles;
     __shared__ uint32_t s_done[kDoneWords];  // batched solves: stopped graphs
@@ -1076,10 +1082,13 @@ __global__ void __launch_bounds__(kBlockThreadsDev) factor_pass_kernel(FactorArg
                 bulk_g2s(st + FS::pos, a.f_pos + gb[2], ns * 4u, bar);
             }
         };
-        produce_tiles<STAGES>(a.thdr, a.f_graph ? a.trange : nullptr, a.tile_list, a.tile_off, a.act_list, a.n_act,
-                              s_done, a.gdone, n_tiles, &ctl->fnext, smem, FS::bytes, full, empty, lane, ctl, fill);
+        produce_tiles<STAGES>(a.thdr, a.f_graph ? a.trange : nullptr, a.dealt, a.per_block, a.act_list, a.n_act, s_done,
+                              a.gdone, n_tiles, &ctl->fnext, smem, FS::bytes, full, empty, lane, ctl, done, fill);
+        // the producer is ahead of its block by now: the sweep's bookkeeping delays no tile
+        if (blockIdx.x == 0 && lane == 0 && !done) sweep_open(ctl, opened);
         return;
     }
+    if (done) return;
 
     {  // factors too large for a tile first, one per block, while the producer's first loads are in flight
         __shared__ typename WideAcc<T>::type s_l[kConsumerWarps];
@@ -1589,8 +1598,7 @@ __global__ void __launch_bounds__(kBlockThreadsDev) var_pass_kernel(VarArgs a, c
     typedef VarStage<T, DAMP> VS;
     constexpr bool RESID = (BMODE == 1 || BMODE == 2 || BMODE == 4);
     constexpr uint32_t psz = sizeof(T) == 4 ? 8u : 16u;
-    if (*(volatile int *)&ctl->done) return;
-    if (blockIdx.x == 0 && threadIdx.x == 0) ctl->fnext = 0u;  // the next factor pass starts after this kernel
+    const int done = *(volatile int *)&ctl->done;  // looked at once the first loads are on their way
     const double pscale = ctl->pscale;
     const double tol = ctl->tol;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -1636,8 +1644,12 @@ __global__ void __launch_bounds__(kBlockThreadsDev) var_pass_kernel(VarArgs a, c
                 if (DAMP) bulk_g2s(st + VS::xo, fvd + gb[2], ns * (uint32_t)sizeof(T), bar);
             }
         };
-        produce_tiles<STAGES>(a.thdr, a.v_graph ? a.trange : nullptr, nullptr, nullptr, a.act_list, a.n_act, s_done,
-                              a.gstate, n_tiles, &ctl->vnext, smem, VS::bytes, full, empty, lane, ctl, fill);
+        produce_tiles<STAGES>(a.thdr, a.v_graph ? a.trange : nullptr, nullptr, 0u, a.act_list, a.n_act, s_done,
+                              a.gstate, n_tiles, &ctl->vnext, smem, VS::bytes, full, empty, lane, ctl, done, fill);
+        if (done) return;
+        if (blockIdx.x == 0 && lane == 0) ctl->fnext = 0u;  // the next factor pass starts after this kernel
+    } else if (done) {
+        return;
     } else {  // consumer warps: variables too large for a tile first
         {  // one per block
             __shared__ typename WideAcc<T>::type s_s[kConsumerWarps];
