@@ -158,7 +158,7 @@ struct flbp_engine {
     // items per block and shared memory.
     int res_plan = -1;
     unsigned res_grid = 1;
-    uint32_t res_rows_f = 0, res_rows_v = 0;
+    uint32_t res_rows_f = 0, res_rows_v = 0, res_huge_blocks = 0;
     size_t res_smem = 0;
     // Cluster run kernel: -1 not planned yet, 0 not for this engine, 1 planned;
     // its cluster size, clusters, rows of items per block, shared memory, jobs
@@ -798,13 +798,28 @@ void plan_resident_t(flbp_engine *e) {
     const uint32_t nfb = L.nf_big - L.nf_huge, nvb = L.nv_big - L.nv_huge;
     const uint32_t n_f = nfb + L.n_fgroups(), n_v = nvb + L.n_vgroups();
     const uint32_t items = std::max({n_f, n_v, 1u}), huge = std::max(L.nf_huge, L.nv_huge);
-    const uint32_t want = std::max((items + 3) / 4, std::max(huge, 1u));
+    // at least two blocks where there are huge factors: some for them, the others for the rest
+    const uint32_t want = std::max({(items + 3) / 4, huge + (L.nf_huge ? 1u : 0u), 1u});
     auto rows = [&](uint32_t n, uint32_t nb) { return (n + nb - 1) / nb; };
     for (int cache = 1; cache >= 0; cache--) {
         // most blocks per SM first
         for (int per = sizeof(T) == 4 ? 2 : 1; per >= 1; per--) {
             const uint32_t nb = std::min<uint32_t>(want, (uint32_t)e->sms * (uint32_t)per);
-            const uint32_t rf = rows(n_f, nb), rv = rows(n_v, nb);
+            // blocks for the factors too large for a tile: their share of the
+            // factor pass's work, a slot of theirs (two log1p or expm1 terms)
+            // counted as 2.2 of the others
+            uint32_t hb = 0;
+            if (L.nf_huge) {
+                double h = 0.0;
+                for (uint32_t b = 0; b < L.nf_huge; b++) h += 2.2 * L.fb_deg[b];
+                const double rest = (double)L.n_active_slots - h / 2.2;
+                hb = (uint32_t)std::min<double>(L.nf_huge, std::max(1.0, std::floor(nb * h / (h + rest) + 0.5)));
+                if (hb >= nb) {  // a block at least for the other items
+                    if (nb < 2) continue;
+                    hb = nb - 1;
+                }
+            }
+            const uint32_t rf = rows(n_f, nb - hb), rv = rows(n_v, nb);
             size_t smem = 0;
             if (cache) {
                 if (rf + rv > kResMaxRows) continue;
@@ -835,6 +850,7 @@ void plan_resident_t(flbp_engine *e) {
             e->res_grid = nb;
             e->res_rows_f = rf;
             e->res_rows_v = rv;
+            e->res_huge_blocks = hb;
             e->res_smem = smem;
             return;
         }
@@ -874,6 +890,7 @@ ResArgs<T> resident_args(flbp_engine *e, int mode, uint32_t cap, bool final_beli
     r.final_beliefs = final_beliefs ? 1 : 0;
     r.rows_f = e->res_rows_f;
     r.rows_v = e->res_rows_v;
+    r.huge_blocks = e->res_huge_blocks;
     return r;
 }
 
