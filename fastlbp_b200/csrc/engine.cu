@@ -828,7 +828,8 @@ void plan_resident_t(flbp_engine *e) {
                     const uint32_t n = fac ? n_f : n_v, big = fac ? nfb : nvb;
                     for (uint32_t j = 0; j < (fac ? rf : rv); j++)
                         for (uint32_t b = 0; b < nb; b++) {
-                            const uint32_t it = res_item_of(j, b, nb);
+                            if (fac && b < hb) continue;
+                            const uint32_t it = fac ? res_item_of(j, b - hb, nb - hb) : res_item_of(j, b, nb);
                             if (it >= n) continue;
                             uint32_t w;
                             if (it < big) {
@@ -1154,6 +1155,7 @@ int launch_run(flbp_engine *e, int kind, int mode, long long cap, bool final_bel
 }
 
 // Stop-rule driven loop: chunks of sweeps until the device sets ctl->done.
+// Leaves the control block of the last chunk in h_ctl.
 int run_loop(flbp_engine *e, int mode, long long cap) {
     long long launched = 0;
     int kind = 0;
@@ -2144,7 +2146,6 @@ int flbp_run_tol(flbp_engine *e, double tol, int64_t maxiter, double maxtime, fl
     long long done_sweeps = 0;
     if (e->iters < maxiter && maxtime > 0.0 && INFINITY > tol) {
         if ((rc = upload_ctl(e)) || (rc = run_loop(e, 1, maxiter - e->iters))) return rc;
-        if ((rc = download_ctl(e))) return rc;
         done_sweeps = e->h_ctl->run_sweeps;
     }
     if ((rc = record_stop(e))) return rc;
@@ -2203,7 +2204,6 @@ int flbp_run_lowpass(flbp_engine *e, double tol, int64_t min_iters, int64_t max_
     long long done_sweeps = 0;
     if (maxtime >= 0.0) {
         if ((rc = upload_ctl(e)) || (rc = run_loop(e, 2, max_iters + 1))) return rc;
-        if ((rc = download_ctl(e))) return rc;
         done_sweeps = e->h_ctl->run_sweeps;
     }
     if (e->h_ctl->reason == FLBP_ALL_CONVERGED && done_sweeps > 0) {
@@ -2706,7 +2706,7 @@ static int run_groups_tol(flbp_engine *e, uint32_t G, double tol, int64_t maxite
             }
         }
         if (open && !over) {
-            if ((rc = run_loop(e, 3, maxiter)) || (rc = download_ctl(e))) return rc;
+            if ((rc = run_loop(e, 3, maxiter))) return rc;
             done_sweeps = std::max<long long>(done_sweeps, e->h_ctl->run_sweeps);
         }
         if (cl) {

@@ -187,7 +187,10 @@ int flbp_kernel_times(flbp_engine *eng, double *ms, int64_t *counts);
  * (every warp of a persistent grid loads its own items straight into
  * registers; 1 = up to 64 registers per thread, two 16-warp blocks per SM,
  * 2 = up to 40 registers, three blocks per SM). Which is faster depends on
- * the graph; new engines start with both passes staged. */
+ * the graph; new engines start with both passes staged. Both forms 0 also let
+ * a run of a graph of up to about a million slots go as one launch that
+ * evaluates the same items in the same order (same results); any other pair
+ * of forms, and flbp_set_kernel_timing, keep the two passes per sweep. */
 typedef struct flbp_tuning {
     int32_t factor_form; /* 0 staged, 1 or 2 direct */
     int32_t var_form;    /* 0 staged, 1 or 2 direct */
