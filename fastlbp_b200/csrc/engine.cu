@@ -1072,11 +1072,21 @@ int plan_cluster_t(flbp_engine *e) {
     e->cl_map_words = (uint32_t)(2 * half);
     e->cl_n_jobs = (uint32_t)jobs.size();
     e->cl_all = jobs.size() == all.size() * copies;
-    int rc;
     const size_t groups = std::max<size_t>({1, e->n_sets, e->n_graphs});
-    if ((rc = dalloc(e, &e->d_cl_jobs, jobs.size())) || (rc = upload(e, e->d_cl_jobs, jobs)) ||
-        (rc = dalloc(e, &e->d_cl_map, (size_t)e->cl_map_words * e->cl_clusters)) || (rc = dalloc(e, &e->d_gdiff, groups)))
-        return rc;
+    const size_t bytes = e->bytes;
+    if (dalloc(e, &e->d_cl_jobs, jobs.size()) || dalloc(e, &e->d_cl_map, (size_t)e->cl_map_words * e->cl_clusters) ||
+        dalloc(e, &e->d_gdiff, groups)) {  // no memory for this kernel's tables: the passes need none
+        cudaGetLastError();
+        dfree(e, e->d_cl_jobs);
+        dfree(e, e->d_cl_map);
+        dfree(e, e->d_gdiff);
+        e->d_cl_jobs = nullptr;
+        e->d_cl_map = nullptr;
+        e->d_gdiff = nullptr;
+        e->bytes = bytes;
+        return FLBP_OK;
+    }
+    if (int rc = upload(e, e->d_cl_jobs, jobs)) return rc;
     FLBP_CUDA(cudaStreamSynchronize(e->stream));  // the job list is a local of this function
     e->cl_plan = 1;
     return FLBP_OK;
@@ -1087,8 +1097,13 @@ int use_cluster(flbp_engine *e, int mode, bool *use) {
     *use = false;
     if (e->seq || e->ktime || e->f_form || e->v_form || e->L.V == 0) return FLBP_OK;
     if ((e->n_sets || e->n_graphs) && mode != 3) return FLBP_OK;
-    if (e->cl_plan < 0)
-        if (int rc = e->prec == 64 ? plan_cluster_t<double>(e) : plan_cluster_t<float>(e)) return rc;
+    if (e->cl_plan < 0) {
+        try {
+            if (int rc = e->prec == 64 ? plan_cluster_t<double>(e) : plan_cluster_t<float>(e)) return rc;
+        } catch (const std::bad_alloc &) {  // not enough host memory to plan: the passes
+            e->cl_plan = 0;
+        }
+    }
     *use = e->cl_plan > 0;
     return FLBP_OK;
 }
