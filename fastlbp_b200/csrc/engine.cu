@@ -2693,8 +2693,16 @@ static int run_groups_tol(flbp_engine *e, uint32_t G, double tol, int64_t maxite
         long long cl_sweeps = 0;
         if (cl) {  // the groups that fit a cluster, each to its own end
             const auto began = std::chrono::steady_clock::now();
+            auto resume = [&]() -> int {  // the control block for a next launch, with the time that is left
+                e->h_ctl->maxtime_ns = maxtime * 1e9 - (double)std::chrono::duration_cast<std::chrono::nanoseconds>(
+                                                           std::chrono::steady_clock::now() - began).count();
+                e->h_ctl->done = 0;
+                std::memset(&e->h_ctl->rs, 0, sizeof(ResSync));
+                return upload_ctl(e);
+            };
             for (bool again = false; open && !over; again = true) {
-                if ((rc = launch_run(e, 2, 3, std::min<long long>(kResSweeps, maxiter), false, again)) ||
+                if ((again && (rc = resume())) ||
+                    (rc = launch_run(e, 2, 3, std::min<long long>(kResSweeps, maxiter), false, false)) ||
                     (rc = download_ctl(e)) || (rc = fetch()))
                     return rc;
                 over = e->h_ctl->done != 0;
@@ -2712,15 +2720,20 @@ static int run_groups_tol(flbp_engine *e, uint32_t G, double tol, int64_t maxite
                 open = n_open > 0;
             }
             done_sweeps = cl_sweeps;
-            open = !e->cl_all;  // the other graphs follow, in the time that is left
-            if (open && !over) {
-                e->h_ctl->maxtime_ns -= (double)std::chrono::duration_cast<std::chrono::nanoseconds>(
-                                            std::chrono::steady_clock::now() - began).count();
-                std::memset(&e->h_ctl->rs, 0, sizeof(ResSync));
-                if ((rc = upload_ctl(e))) return rc;
+            // the other graphs follow in the time that is left, with one sweep at least
+            open = !e->cl_all;
+            if (open && over) {  // out of time: the ones of the clusters have ended
+                for (uint32_t g = 0; g < G; g++)
+                    if (st[2 * (size_t)G + g] && !st[g]) {
+                        st[g] = 1;
+                        st[3 * (size_t)G + g] = FLBP_DIVERGED;
+                    }
+                FLBP_CUDA(cudaMemcpyAsync(e->d_gstate, st.data(), st.size() * sizeof(int), cudaMemcpyHostToDevice, e->stream));
+                FLBP_CUDA(cudaStreamSynchronize(e->stream));
             }
+            if (open && (rc = resume())) return rc;
         }
-        if (open && !over) {
+        if (open) {
             if ((rc = run_loop(e, 3, maxiter))) return rc;
             done_sweeps = std::max<long long>(done_sweeps, e->h_ctl->run_sweeps);
         }
@@ -2728,7 +2741,7 @@ static int run_groups_tol(flbp_engine *e, uint32_t G, double tol, int64_t maxite
             if ((rc = fetch())) return rc;
             if (cl_sweeps > e->h_ctl->run_sweeps) e->h_ctl->maxdiff = cl_diff;
             else if (cl_sweeps == e->h_ctl->run_sweeps) e->h_ctl->maxdiff = std::max(e->h_ctl->maxdiff, cl_diff);
-            bool all = true;
+            bool all = !over;
             for (uint32_t g = 0; g < G; g++) all &= st[g] != 0;
             e->h_ctl->reason = all ? FLBP_ALL_CONVERGED : FLBP_DIVERGED;
         }

@@ -149,3 +149,28 @@ def test_batch_continued_and_limited():
         got.append([*one, *two, e.beliefs(), [info["sweeps"], info["reason"], info["maxdiff"]], *e.vf_messages()])
     _equal(got[0], got[1], "continued")
     e.close()
+
+
+@pytest.mark.parametrize("prec", [32, 64])
+def test_batch_out_of_time(prec):
+    """No time at all: one sweep of every graph, the ones too large for a cluster too."""
+    graphs = [_bingo(n, seed=n) for n in (20, 300, 90)] + [_large()]
+    e = BatchEngine(graphs, precision=prec)
+    got = []
+    for timed in (False, True):
+        e.set_kernel_timing(timed)
+        e.reset_counts()
+        e.init()
+        sweeps, reasons = e.run_batch_tol(1e-9, 30, 1e-9)
+        assert np.all(np.asarray(sweeps) == 1)
+        got.append([e.beliefs(), reasons, [e.info.as_dict()["reason"]], *e.vf_messages()])
+    _equal(got[0], got[1], "out of time")
+    e.close()
+
+
+def test_batch_time_over_several_launches():
+    """The time limit counts from the call, not from a launch of 4,096 sweeps."""
+    e = BatchEngine([_bingo(n, seed=n) for n in (20, 90)])
+    sweeps, _ = e.run_batch_tol(-1.0, 400_000, 0.1)  # no belief is ever settled
+    assert np.all((np.asarray(sweeps) > 4096) & (np.asarray(sweeps) < 400_000))
+    e.close()
