@@ -163,6 +163,11 @@ __global__ void __launch_bounds__(kClusterThreads<T>, 1) cluster_kernel(ClusterA
     uint32_t *map = r.map + (size_t)cid * r.map_words;
     const T *pqg = reinterpret_cast<const T *>(r.f.f_pq);
     if (tid == 0) s_over = 0;
+    // A block's shared memory may be written by the others only once it has
+    // started: blocks of a cluster are scheduled together, not started
+    // together. (One barrier per launch; it also orders s_over's first value
+    // before any remote store to it.)
+    cluster_sync_all();
 
     for (;;) {
         // ---- the next job of the queue, for the whole cluster
