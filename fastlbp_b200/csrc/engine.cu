@@ -2680,11 +2680,11 @@ static int run_groups_tol(flbp_engine *e, uint32_t G, double tol, int64_t maxite
     if ((rc = record_start(e))) return rc;
     long long done_sweeps = 0;
     std::vector<int> st(4 * (size_t)G);
-    auto fetch = [&]() -> int {
+    auto queue_fetch = [&]() -> int {
         FLBP_CUDA(cudaMemcpyAsync(st.data(), e->d_gstate, st.size() * sizeof(int), cudaMemcpyDeviceToHost, e->stream));
-        FLBP_CUDA(cudaStreamSynchronize(e->stream));
         return FLBP_OK;
     };
+    bool fresh = false;  // st is the groups' state at the end of the run
     if (maxiter > 0 && maxtime > 0.0) {
         if ((rc = upload_ctl(e))) return rc;
         bool cl = false, over = false, open = true;
@@ -2700,14 +2700,16 @@ static int run_groups_tol(flbp_engine *e, uint32_t G, double tol, int64_t maxite
                 std::memset(&e->h_ctl->rs, 0, sizeof(ResSync));
                 return upload_ctl(e);
             };
+            std::vector<double> diff(G);
             for (bool again = false; open && !over; again = true) {
                 if ((again && (rc = resume())) ||
-                    (rc = launch_run(e, 2, 3, std::min<long long>(kResSweeps, maxiter), false, false)) ||
-                    (rc = download_ctl(e)) || (rc = fetch()))
+                    (rc = launch_run(e, 2, 3, std::min<long long>(kResSweeps, maxiter), false, false)))
                     return rc;
+                // in the order of the engine's stream, like every other copy: nothing here waits for work
+                // on the process's default stream
+                FLBP_CUDA(cudaMemcpyAsync(diff.data(), e->d_gdiff, G * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
+                if ((rc = queue_fetch()) || (rc = download_ctl(e))) return rc;
                 over = e->h_ctl->done != 0;
-                std::vector<double> diff(G);
-                FLBP_CUDA(cudaMemcpy(diff.data(), e->d_gdiff, G * sizeof(double), cudaMemcpyDeviceToHost));
                 uint32_t n_open = 0;
                 cl_sweeps = 0;
                 cl_diff = 0.0;
@@ -2737,8 +2739,13 @@ static int run_groups_tol(flbp_engine *e, uint32_t G, double tol, int64_t maxite
             if ((rc = run_loop(e, 3, maxiter))) return rc;
             done_sweeps = std::max<long long>(done_sweeps, e->h_ctl->run_sweeps);
         }
+        fresh = cl && !open;
         if (cl) {
-            if ((rc = fetch())) return rc;
+            if (!fresh) {
+                if ((rc = queue_fetch())) return rc;
+                FLBP_CUDA(cudaStreamSynchronize(e->stream));
+                fresh = true;
+            }
             if (cl_sweeps > e->h_ctl->run_sweeps) e->h_ctl->maxdiff = cl_diff;
             else if (cl_sweeps == e->h_ctl->run_sweeps) e->h_ctl->maxdiff = std::max(e->h_ctl->maxdiff, cl_diff);
             bool all = !over;
@@ -2746,7 +2753,11 @@ static int run_groups_tol(flbp_engine *e, uint32_t G, double tol, int64_t maxite
             e->h_ctl->reason = all ? FLBP_ALL_CONVERGED : FLBP_DIVERGED;
         }
     }
-    if ((rc = record_stop(e)) || (rc = fetch())) return rc;
+    if ((rc = record_stop(e))) return rc;
+    if (!fresh) {
+        if ((rc = queue_fetch())) return rc;
+        FLBP_CUDA(cudaStreamSynchronize(e->stream));
+    }
     for (uint32_t g = 0; g < G; g++) {
         if (sweeps) sweeps[g] = st[2 * (size_t)G + g];
         if (reasons) reasons[g] = st[g] ? st[3 * (size_t)G + g] : FLBP_DIVERGED;
