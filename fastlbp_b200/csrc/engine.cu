@@ -804,7 +804,7 @@ void plan_resident_t(flbp_engine *e) {
     for (int cache = 1; cache >= 0; cache--) {
         // most blocks per SM first
         for (int per = sizeof(T) == 4 ? 2 : 1; per >= 1; per--) {
-            const uint32_t nb = std::min<uint32_t>(want, (uint32_t)e->sms * (uint32_t)per);
+            const uint32_t nb = std::min({want, (uint32_t)e->sms * (uint32_t)per, kResMaxBlocks});
             // blocks for the factors too large for a tile: their share of the
             // factor pass's work, a slot of theirs (two log1p or expm1 terms)
             // counted as 2.2 of the others

@@ -42,17 +42,19 @@ constexpr int kGroupWords = 128;  // groups that stop by themselves in one resid
 struct ResSync {
     unsigned int arrive;  // block arrivals at the barriers between the passes, over the whole launch
     unsigned int pad[3];
-    // Per slot, one 16-byte word read at once by the barrier that ends a
-    // sweep: max |belief change| (double bits); blocks arrived, with
-    // kResTimeUp added once the run's time is over.
-    struct alignas(16) End {
+    // Per slot: max |belief change| (double bits), and the word that the
+    // barrier which ends a sweep polls: the blocks that have arrived, plus
+    // kResMoved for each of them with a change above the tolerance, plus
+    // kResTimeUp once the run's time is over.
+    struct End {
         unsigned long long maxdiff;
         unsigned int arrive, pad;
     } end[3];
     unsigned long long nonconv[3];
     unsigned int moved[3][kGroupWords];
 };
-constexpr unsigned int kResTimeUp = 1u << 24;
+constexpr unsigned int kResMoved = 1u << 12, kResTimeUp = 1u << 24;
+constexpr unsigned int kResMaxBlocks = kResMoved - 1u;  // both counts of an end word have 12 bits
 
 struct Ctl {
     unsigned long long maxdiff_bits;  // max |belief change| of this sweep, double bits

@@ -102,24 +102,17 @@ __device__ __forceinline__ bool res_arrive_wait(unsigned int *arrive, unsigned i
     }
 }
 
-// The same at the end of a sweep, on the slot's 16-byte word: block 0 adds
-// kResTimeUp when the run's time is over. Each block's residual went into the
-// word before its arrival, so the word that shows all arrivals holds the
-// sweep's residual.
-__device__ __forceinline__ bool res_end_wait(ResSync::End *w, unsigned int nb, bool time_up,
-                                             unsigned long long &maxdiff_bits, bool &over) {
-    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(&w->arrive), "r"(1u + (time_up ? kResTimeUp : 0u))
-                 : "memory");
+// The same at the end of a sweep, on the slot's end word, to which a block
+// adds 1, kResMoved and kResTimeUp as they apply. What the stop rule needs of
+// the other blocks is in the word that is polled, so that no further load
+// follows the barrier; releases and acquire are 32-bit accesses of the one
+// word, and order the residuals and messages of all blocks.
+__device__ __forceinline__ bool res_end_wait(unsigned int *arrive, unsigned int nb, unsigned int add,
+                                             unsigned int &word) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(arrive), "r"(add) : "memory");
     auto opened = [&]() {
-        unsigned long long lo, hi;
-        asm volatile(
-            "{\n\t.reg .b128 v;\n\tld.acquire.gpu.global.b128 v, [%2];\n\tmov.b128 {%0, %1}, v;\n\t}"
-            : "=l"(lo), "=l"(hi)
-            : "l"(w)
-            : "memory");
-        maxdiff_bits = lo;
-        over = ((unsigned int)hi & kResTimeUp) != 0;
-        return ((unsigned int)hi & (kResTimeUp - 1u)) == nb;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(word) : "l"(arrive) : "memory");
+        return (word & (kResMoved - 1u)) == nb;
     };
     if (opened()) return true;
     const long long t0 = clock64();
@@ -480,7 +473,7 @@ __global__ void __launch_bounds__(kResThreads, sizeof(T) == 4 ? 2 : 1) resident_
             if (s_moved[w]) atomicOr(&rs->moved[slot][w], s_moved[w]);
         if (gwords) __syncthreads();
         if (wid == 0) {
-            bool time_up = false;
+            unsigned int add = 1u;
             if (mode) {
                 double m = warp_max(lane < kConsumerWarps ? s_max[lane] : 0.0);
                 unsigned long long c = 0;
@@ -488,28 +481,28 @@ __global__ void __launch_bounds__(kResThreads, sizeof(T) == 4 ? 2 : 1) resident_
                 if (lane == 0) {
                     if (m > 0.0) atomicMax(&rs->end[slot].maxdiff, (unsigned long long)__double_as_longlong(m));
                     if (c) atomicAdd(&rs->nonconv[slot], c);
+                    if (m > tol) add += kResMoved;
                     if (b == 0) {
                         unsigned long long now;
                         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
                         const double elapsed = (double)(now - t_start);
-                        time_up = mode == 2 ? elapsed > maxtime_ns : elapsed >= maxtime_ns;
+                        if (mode == 2 ? elapsed > maxtime_ns : elapsed >= maxtime_ns) add += kResTimeUp;
                     }
                 }
             }
-            unsigned long long bits = 0;
-            bool over = false;
-            if (lane == 0 && !res_end_wait(&rs->end[slot], nb, time_up, bits, over)) {
+            unsigned int word = 0;
+            if (lane == 0 && !res_end_wait(&rs->end[slot].arrive, nb, add, word)) {
                 s_stop = 2;
             } else if (lane == 0 && mode) {
-                maxdiff_bits = bits;
-                maxdiff = __longlong_as_double((long long)bits);
+                const bool over = (word & kResTimeUp) != 0, moved = (word & (kResTimeUp - kResMoved)) != 0;
                 const long long n = run0 + (long long)s + 1;
                 if (mode == 1) {  // the rules of stop_rules
-                    if (!(iters0 + n < maxiter && maxdiff > tol && !over)) {
+                    if (!(iters0 + n < maxiter && moved && !over)) {
                         s_stop = 1;
-                        reason = (maxdiff > tol) ? FLBP_DIVERGED : FLBP_ALL_CONVERGED;
+                        reason = moved ? FLBP_DIVERGED : FLBP_ALL_CONVERGED;
                     }
                 } else if (mode == 2) {
+                    maxdiff = __longlong_as_double((long long)__ldcg(&rs->end[slot].maxdiff));
                     nonconv = __ldcg(&rs->nonconv[slot]);
                     frac = (double)nonconv / n_vars;
                     if (n >= min_iters) node_frac_tol = (double)(n - min_iters) / (double)(max_iters - min_iters);
@@ -576,6 +569,10 @@ __global__ void __launch_bounds__(kResThreads, sizeof(T) == 4 ? 2 : 1) resident_
         return;
     }
     if (b == 0 && tid == 0) {
+        if (mode) {  // the last sweep's residual: its slot is cleared two sweeps later at the earliest
+            maxdiff_bits = __ldcg(&rs->end[(s - 1u) % 3u].maxdiff);
+            maxdiff = __longlong_as_double((long long)maxdiff_bits);
+        }
         ctl->t = t0 + (long long)s;
         ctl->run_sweeps = run0 + (long long)s;
         ctl->t_start_ns = t_start;
