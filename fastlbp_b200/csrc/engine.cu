@@ -175,6 +175,7 @@ struct flbp_engine {
     std::vector<uint8_t> batch_huge;     // and whether it has items too large for a tile
     uint32_t *d_cut_ent = nullptr;       // sets: cut entries as bits (per set)
     uint32_t cut_words = 0;
+    int refuse_launches = 0;             // flbp_test_refuse_launches
     std::map<std::pair<int, int>, cudaGraphExec_t> graphs;  // (mode, sweeps) -> executable graph
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     float last_ms = 0.f;
@@ -1153,18 +1154,37 @@ int run_kernel(flbp_engine *e, int mode, int *kind) {
     return FLBP_OK;
 }
 
+// A launch of a whole run that CUDA will not make here: the stream's context
+// has fewer SMs or less room than the plan counted on. Nothing has run then,
+// and the pass kernels need no such room. Clears the error.
+bool launch_refused(cudaError_t c) {
+    if (c != cudaErrorCooperativeLaunchTooLarge && c != cudaErrorLaunchOutOfResources &&
+        c != cudaErrorInvalidConfiguration && c != cudaErrorInvalidClusterSize && c != cudaErrorNotSupported)
+        return false;
+    cudaGetLastError();
+    return true;
+}
+
 // At most `cap` (<= kResSweeps) sweeps of a mode in one launch of such a
 // kernel; `again`: not the first launch after the control block's upload.
-int launch_run(flbp_engine *e, int kind, int mode, long long cap, bool final_beliefs, bool again) {
+// Where the launch is refused, *refused is set and the engine's later runs
+// don't plan for this kernel any more.
+int launch_run(flbp_engine *e, int kind, int mode, long long cap, bool final_beliefs, bool again, bool *refused) {
+    *refused = false;
     if (again)
         FLBP_CUDA(cudaMemsetAsync(reinterpret_cast<char *>(e->d_ctl) + offsetof(Ctl, rs), 0, sizeof(ResSync), e->stream));
     const uint32_t n = (uint32_t)cap;
-    if (kind == 2)
-        FLBP_CUDA(e->prec == 64 ? launch_cluster_t<double>(e, mode, n, final_beliefs)
-                                : launch_cluster_t<float>(e, mode, n, final_beliefs));
-    else
-        FLBP_CUDA(e->prec == 64 ? launch_resident_t<double>(e, mode, n, final_beliefs)
-                                : launch_resident_t<float>(e, mode, n, final_beliefs));
+    const cudaError_t c = e->refuse_launches > 0 ? (e->refuse_launches--, cudaErrorCooperativeLaunchTooLarge)
+                          : kind == 2 ? (e->prec == 64 ? launch_cluster_t<double>(e, mode, n, final_beliefs)
+                                                       : launch_cluster_t<float>(e, mode, n, final_beliefs))
+                          : e->prec == 64 ? launch_resident_t<double>(e, mode, n, final_beliefs)
+                                          : launch_resident_t<float>(e, mode, n, final_beliefs);
+    if (launch_refused(c)) {
+        (kind == 2 ? e->cl_plan : e->res_plan) = 0;
+        *refused = true;
+        return FLBP_OK;
+    }
+    FLBP_CUDA(c);
     e->launches += 1;
     return FLBP_OK;
 }
@@ -1174,17 +1194,24 @@ int launch_run(flbp_engine *e, int kind, int mode, long long cap, bool final_bel
 int run_loop(flbp_engine *e, int mode, long long cap) {
     long long launched = 0;
     int kind = 0;
-    if (mode == 3) kind = use_resident(e, mode) ? 1 : 0;  // run_groups_tol has called the cluster kernel
-    else if (int rc = run_kernel(e, mode, &kind)) return rc;
-    if (kind) {
-        while (launched < cap) {
-            const long long n = std::min<long long>(kResSweeps, cap - launched);
-            int rc = launch_run(e, kind, mode, n, false, launched > 0);
-            if (rc || (rc = download_ctl(e))) return rc;
-            launched += n;
-            if (e->h_ctl->done) break;
-        }
+    auto choose = [&]() -> int {
+        if (mode != 3) return run_kernel(e, mode, &kind);
+        kind = use_resident(e, mode) ? 1 : 0;  // run_groups_tol has called the cluster kernel
         return FLBP_OK;
+    };
+    if (int rc = choose()) return rc;
+    while (kind && launched < cap) {
+        const long long n = std::min<long long>(kResSweeps, cap - launched);
+        bool refused;
+        int rc = launch_run(e, kind, mode, n, false, launched > 0, &refused);
+        if (rc) return rc;
+        if (refused) {
+            if ((rc = choose())) return rc;
+            continue;
+        }
+        if ((rc = download_ctl(e))) return rc;
+        launched += n;
+        if (e->h_ctl->done) return FLBP_OK;
     }
     int k = 1;
     while (launched < cap) {
@@ -2114,14 +2141,16 @@ int flbp_run_fixed(flbp_engine *e, int64_t sweeps, flbp_run_info *info) {
     if ((rc = record_start(e)) || (rc = upload_ctl(e))) return rc;
     int kind = 0;
     if (sweeps > 0 && (rc = run_kernel(e, 0, &kind))) return rc;
-    if (kind) {
-        for (long long left = sweeps; left > 0;) {
-            const long long n = std::min<long long>(kResSweeps, left);
-            if ((rc = launch_run(e, kind, 0, n, n == left, left < sweeps))) return rc;
-            left -= n;
-        }
-    } else {
-        if ((rc = launch_sweeps(e, 0, sweeps))) return rc;
+    long long left = sweeps;
+    while (kind && left > 0) {
+        const long long n = std::min<long long>(kResSweeps, left);
+        bool refused;
+        if ((rc = launch_run(e, kind, 0, n, n == left, left < sweeps, &refused))) return rc;
+        if (!refused) left -= n;
+        else if ((rc = run_kernel(e, 0, &kind))) return rc;
+    }
+    if (!kind) {
+        if ((rc = launch_sweeps(e, 0, left))) return rc;
         launch_beliefs_only(e, e->d_belief);
     }
     FLBP_CUDA(cudaMemcpyAsync(e->d_lowpass, e->d_belief, std::max<size_t>(1, e->L.V) * sizeof(double),
@@ -2651,6 +2680,15 @@ int flbp_engine_layout_digest(flbp_engine *e, uint64_t *digest, int32_t *built_o
     return FLBP_OK;
 }
 
+// For tests of the way back to the pass kernels: the engine's next n launches
+// of a whole run return an error code instead of being made.
+int flbp_test_refuse_launches(flbp_engine *e, int32_t n) {
+    int rc = begin_call(e);
+    if (rc) return rc;
+    e->refuse_launches = n;
+    return FLBP_OK;
+}
+
 int flbp_last_run_ms(flbp_engine *e, double *ms) {
     if (!e || !ms) {
         set_error("null argument");
@@ -2702,9 +2740,18 @@ static int run_groups_tol(flbp_engine *e, uint32_t G, double tol, int64_t maxite
             };
             std::vector<double> diff(G);
             for (bool again = false; open && !over; again = true) {
+                bool refused;
                 if ((again && (rc = resume())) ||
-                    (rc = launch_run(e, 2, 3, std::min<long long>(kResSweeps, maxiter), false, false)))
+                    (rc = launch_run(e, 2, 3, std::min<long long>(kResSweeps, maxiter), false, false, &refused)))
                     return rc;
+                if (refused && again) {  // its groups are on the way: the passes count a run's sweeps from its start
+                    set_error("a continued cluster launch was refused");
+                    return FLBP_ERR_CUDA;
+                }
+                if (refused) {
+                    cl = false;
+                    break;
+                }
                 // in the order of the engine's stream, like every other copy: nothing here waits for work
                 // on the process's default stream
                 FLBP_CUDA(cudaMemcpyAsync(diff.data(), e->d_gdiff, G * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
@@ -2723,7 +2770,7 @@ static int run_groups_tol(flbp_engine *e, uint32_t G, double tol, int64_t maxite
             }
             done_sweeps = cl_sweeps;
             // the other graphs follow in the time that is left, with one sweep at least
-            open = !e->cl_all;
+            if (cl) open = !e->cl_all;
             if (open && over) {  // out of time: the ones of the clusters have ended
                 for (uint32_t g = 0; g < G; g++)
                     if (st[2 * (size_t)G + g] && !st[g]) {
@@ -2733,7 +2780,7 @@ static int run_groups_tol(flbp_engine *e, uint32_t G, double tol, int64_t maxite
                 FLBP_CUDA(cudaMemcpyAsync(e->d_gstate, st.data(), st.size() * sizeof(int), cudaMemcpyHostToDevice, e->stream));
                 FLBP_CUDA(cudaStreamSynchronize(e->stream));
             }
-            if (open && (rc = resume())) return rc;
+            if (cl && open && (rc = resume())) return rc;
         }
         if (open) {
             if ((rc = run_loop(e, 3, maxiter))) return rc;
@@ -2969,25 +3016,30 @@ char *adj_seg_fv(flbp_engine *e, long long i) {
 template <typename T>
 int adjoint_sweeps(flbp_engine *e, long long n, const T *v0, T *vseg, size_t vstride, T *fseg, size_t fstride,
                    T *vlast) {
-    if (use_resident(e, 1)) {  // up to the larger limit: without it every sweep is two launches that no graph replays
-        for (long long i = 0; i < n; i += kResSweeps) {
-            const long long m = std::min<long long>(kResSweeps, n - i);
-            ResArgs<T> r = resident_args<T>(e, 0, (uint32_t)m, false);
-            r.states = 1;
-            r.v0 = i == 0 ? v0 : vseg + (size_t)i * vstride;
-            r.vseg = vseg + (size_t)i * vstride;
-            r.fseg = fseg + (size_t)i * fstride;
-            r.vstride = vstride;
-            r.fstride = fstride;
-            r.vlast = i + m < n ? r.vseg + (size_t)m * vstride : vlast;
-            FLBP_CUDA(cudaMemsetAsync(reinterpret_cast<char *>(e->d_ctl) + offsetof(Ctl, rs), 0, sizeof(ResSync),
-                                      e->stream));
-            FLBP_CUDA(resident_launch<T>(false, e->res_plan == 2, e->res_grid, e->res_smem, r, e->stream));
-            e->launches += 1;
+    long long i = 0;
+    // up to the larger limit: without it every sweep is two launches that no graph replays
+    for (; i < n && use_resident(e, 1); i += kResSweeps) {
+        const long long m = std::min<long long>(kResSweeps, n - i);
+        ResArgs<T> r = resident_args<T>(e, 0, (uint32_t)m, false);
+        r.states = 1;
+        r.v0 = i == 0 ? v0 : vseg + (size_t)i * vstride;
+        r.vseg = vseg + (size_t)i * vstride;
+        r.fseg = fseg + (size_t)i * fstride;
+        r.vstride = vstride;
+        r.fstride = fstride;
+        r.vlast = i + m < n ? r.vseg + (size_t)m * vstride : vlast;
+        FLBP_CUDA(cudaMemsetAsync(reinterpret_cast<char *>(e->d_ctl) + offsetof(Ctl, rs), 0, sizeof(ResSync), e->stream));
+        const cudaError_t c = e->refuse_launches > 0
+                                  ? (e->refuse_launches--, cudaErrorCooperativeLaunchTooLarge)
+                                  : resident_launch<T>(false, e->res_plan == 2, e->res_grid, e->res_smem, r, e->stream);
+        if (launch_refused(c)) {
+            e->res_plan = 0;
+            break;
         }
-        return FLBP_OK;
+        FLBP_CUDA(c);
+        e->launches += 1;
     }
-    for (long long i = 0; i < n; i++) {
+    for (; i < n; i++) {
         T *vout = i + 1 < n ? vseg + (size_t)(i + 1) * vstride : vlast;
         launch_factor_pass_on<T>(e, i == 0 ? v0 : vseg + (size_t)i * vstride, fseg + (size_t)i * fstride);
         if (vout) launch_var_pass_on<T>(e, fseg + (size_t)i * fstride, vout);
