@@ -160,6 +160,7 @@ struct flbp_engine {
     unsigned res_grid = 1;
     uint32_t res_rows_f = 0, res_rows_v = 0, res_huge_blocks = 0;
     size_t res_smem = 0;
+    int64_t n_bare = -1;  // variables without entries (bare_vars), -1: not counted yet
     // Cluster run kernel: -1 not planned yet, 0 not for this engine, 1 planned;
     // its cluster size, clusters, rows of items per block, shared memory, jobs
     // (device) and position maps.
@@ -786,6 +787,19 @@ constexpr long long kResSweeps = 4096;  // sweeps per launch at most
 // 18.1 : 19.4 at 709 k, 19.6 : 18.9 at 952 k. FP64 crosses at the same sizes.
 constexpr uint64_t kResFixedSlots = 720000, kResRuleSlots = 980000;
 
+// Variables without entries among variable groups [g0, g1): a sweep that
+// takes beliefs reads a prior and reads and writes a belief for each.
+uint64_t bare_vars(const HostLayout &L, uint32_t g0, uint32_t g1) {
+    uint64_t n = 0;
+    for (uint32_t g = g0; g < g1; g++) n += L.vg_base[g + 1] == L.vg_base[g] ? 32 : 0;
+    return n;
+}
+
+uint64_t bare_vars(flbp_engine *e) {
+    if (e->n_bare < 0) e->n_bare = (int64_t)bare_vars(e->L, 0, e->L.n_vgroups());
+    return (uint64_t)e->n_bare;
+}
+
 // Grid, rows and shared memory of the resident kernel for this engine's
 // graph, or a plan of 0 where the pass kernels run instead.
 template <typename T>
@@ -863,7 +877,13 @@ void plan_resident_t(flbp_engine *e) {
 // per-pass timing, a parallel schedule and a graph of its range.
 bool use_resident(flbp_engine *e, int mode) {
     if (e->seq || e->ktime || e->f_form || e->v_form || e->L.V == 0 || e->n_sets) return false;
-    if (e->L.n_slots > (mode == 0 ? kResFixedSlots : kResRuleSlots)) return false;
+    // A variable without entries costs the resident kernel more than the passes, whose blocks come in
+    // waves: as much as a slot does in fixed runs, half of that with a tolerance, a quarter in low-pass
+    // runs. Measured, passes against resident, ms of a run on 83 k slots: 50 fixed sweeps 0.66 : 0.57 with
+    // 0.3 M of them, 0.80 : 0.86 with 1 M; to 1e-6 0.96 : 0.75 with 1 M, 1.33 : 1.62 with 3 M; low-pass
+    // 2.17 : 1.34 with 3 M, 3.1 : 3.2 with 6 M.
+    const uint64_t bare = bare_vars(e) / (mode == 0 ? 1 : mode == 2 ? 4 : 2);
+    if (e->L.n_slots + bare > (mode == 0 ? kResFixedSlots : kResRuleSlots)) return false;
     if (e->res_plan < 0) {
         if (e->prec == 64) plan_resident_t<double>(e);
         else plan_resident_t<float>(e);
@@ -909,6 +929,9 @@ cudaError_t launch_resident_t(flbp_engine *e, int mode, uint32_t cap, bool final
 // per tolerance sweep against the resident kernel: FP32 6.1 : 9.3 us at 4 k
 // slots, 7.4 : 9.5 at 24 k, 9.7 : 10.2 at 40 k, 12.0 : 10.4 at 63 k; FP64
 // 10.1 : 11.4 at 12 k, 11.1 : 11.1 at 24 k, 15.6 : 11.6 at 40 k.
+// A variable without entries counts as half a slot: to 1e-6 on 21 k slots,
+// resident against cluster, 0.40 : 0.36 ms with 20 k of them, 0.40 : 0.59 with
+// 100 k, 0.50 : 1.13 with 300 k.
 constexpr uint64_t kClusterSlots32 = 42000, kClusterSlots64 = 18000;
 
 // A job's items in shared-memory words: all of them, and the largest one.
@@ -975,7 +998,8 @@ int plan_cluster_t(flbp_engine *e) {
         all = e->batch_jobs;
         huge = e->batch_huge;
     } else {
-        if (!e->n_sets && L.n_slots > (sizeof(T) == 4 ? kClusterSlots32 : kClusterSlots64)) return FLBP_OK;
+        if (!e->n_sets && L.n_slots + bare_vars(e) / 2 > (sizeof(T) == 4 ? kClusterSlots32 : kClusterSlots64))
+            return FLBP_OK;
         ClusterJob J = {};
         J.fg1 = L.n_fgroups();
         J.f_hi = L.nf_sell;
@@ -993,7 +1017,7 @@ int plan_cluster_t(flbp_engine *e) {
     auto items_v = [](const ClusterJob &J) { return J.vb1 - J.vb0 + J.vg1 - J.vg0; };
     auto job_slots = [&](const ClusterJob &J) {
         return (uint64_t)(L.fg_base[J.fg1] - L.fg_base[J.fg0]) +
-               (J.fb1 > J.fb0 ? (uint64_t)(L.fb_off[J.fb1] - L.fb_off[J.fb0]) : 0u);
+               (J.fb1 > J.fb0 ? (uint64_t)(L.fb_off[J.fb1] - L.fb_off[J.fb0]) : 0u) + bare_vars(L, J.vg0, J.vg1) / 2;
     };
     std::vector<ClusterLoad> load(all.size());
     for (size_t k = 0; k < all.size(); k++)
