@@ -1701,31 +1701,33 @@ __global__ void __launch_bounds__(kBlockThreadsDev) var_pass_kernel(VarArgs a, c
                 A S0 = AccOps<A>::zero();
                 int npos = 0, nneg = 0;
                 if (v < a.nv_sell) decode_prior<T>(st + VS::prior, t, pscale, S0, npos, nneg);
-                // as if every message were finite (padding entries hold 0): a finite sum then was right
                 A S = S0;
-                for (int k = 0; k < wl; k++) {
-                    const int i = 32 * k + lane;
-                    AccOps<A>::add(S, take_fv_fin<T, DAMP>(x[i], DAMP ? xo[i] : T(0), d));
-                }
-                // One send loop for both cases (a lane's own by its condition costs the warp both: 40 damped
-                // sweeps of 1.7 M slots with clamped variables 1.28 ms that way, 1.21 so).
-                if (!AccOps<A>::finite(S)) {  // exact zeros among the messages: counted apart
-                    S = S0;
+                if (w) {  // variables with entries
+                    // as if every message were finite (padding entries hold 0): a finite sum then was right
+                    for (int k = 0; k < wl; k++) {
+                        const int i = 32 * k + lane;
+                        AccOps<A>::add(S, take_fv_fin<T, DAMP>(x[i], DAMP ? xo[i] : T(0), d));
+                    }
+                    // One send loop for both cases (a lane's own by its condition costs the warp both: 40 damped
+                    // sweeps of 1.7 M slots with clamped variables 1.28 ms that way, 1.21 so).
+                    if (!AccOps<A>::finite(S)) {  // exact zeros among the messages: counted apart
+                        S = S0;
+                        for (int k = 0; k < wl; k++) {
+                            const int i = 32 * k + lane;
+                            const T xv = take_fv<T, DAMP>(x[i], DAMP ? xo[i] : T(0), d);
+                            if (xv == inf) npos++;
+                            else if (xv == -inf) nneg++;
+                            else AccOps<A>::add(S, xv);
+                        }
+                    }
                     for (int k = 0; k < wl; k++) {
                         const int i = 32 * k + lane;
                         const T xv = take_fv<T, DAMP>(x[i], DAMP ? xo[i] : T(0), d);
-                        if (xv == inf) npos++;
-                        else if (xv == -inf) nneg++;
-                        else AccOps<A>::add(S, xv);
-                    }
-                }
-                for (int k = 0; k < wl; k++) {
-                    const int i = 32 * k + lane;
-                    const T xv = take_fv<T, DAMP>(x[i], DAMP ? xo[i] : T(0), d);
-                    if (DAMP) fvd[gb[2] + base + i] = xv;
-                    if (WRITE_VF) {
-                        const uint32_t e = en[i];
-                        if (e != kSentinel) vf[e] = excl_msg<T>(S, npos, nneg, xv);
+                        if (DAMP) fvd[gb[2] + base + i] = xv;
+                        if (WRITE_VF) {
+                            const uint32_t e = en[i];
+                            if (e != kSentinel) vf[e] = excl_msg<T>(S, npos, nneg, xv);
+                        }
                     }
                 }
                 if (v < a.nv_sell && live) {
