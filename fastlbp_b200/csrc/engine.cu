@@ -784,8 +784,16 @@ constexpr long long kResSweeps = 4096;  // sweeps per launch at most
 // graphs): tolerance runs 11.1 : 18.3 us at 158 k slots, 17.4 : 23.9 at
 // 635 k, 22.3 : 26.7 at 952 k but 29.3 : 27.0 with fan-ins up to 4,096 at
 // 1.0 M; fixed runs, which have no residual to reduce, 9.2 : 11.2 at 158 k,
-// 18.1 : 19.4 at 709 k, 19.6 : 18.9 at 952 k. FP64 crosses at the same sizes.
-constexpr uint64_t kResFixedSlots = 720000, kResRuleSlots = 980000;
+// 16.3 : 18.5 at 698 k, 19.6 : 18.9 at 952 k but 21.1 : 20.4 with fan-ins up
+// to 4,096 at 710 k.
+constexpr uint64_t kResFixedSlots = 700000, kResRuleSlots = 980000;
+// In FP64 and damped fixed runs a factor that takes a warp (its block waits
+// for it at the barrier) costs the resident kernel the more: its slots count
+// seven times. Measured per sweep, passes against resident, graphs with 12 %
+// of their slots in such factors: FP64 32.1 : 30.9 us at 354 k slots, 33.7 :
+// 35.6 damped at 473 k, 37.7 : 40.4 at 590 k; FP32 damped 17.6 : 16.3, 17.6 :
+// 18.4 and 19.7 : 19.4; without such factors FP64 29.4 : 21.5 at 698 k.
+constexpr uint64_t kResWarpSlot = 6;
 
 // Variables without entries among variable groups [g0, g1): a sweep that
 // takes beliefs reads a prior and reads and writes a belief for each.
@@ -882,8 +890,10 @@ bool use_resident(flbp_engine *e, int mode) {
     // runs. Measured, passes against resident, ms of a run on 83 k slots: 50 fixed sweeps 0.66 : 0.57 with
     // 0.3 M of them, 0.80 : 0.86 with 1 M; to 1e-6 0.96 : 0.75 with 1 M, 1.33 : 1.62 with 3 M; low-pass
     // 2.17 : 1.34 with 3 M, 3.1 : 3.2 with 6 M.
-    const uint64_t bare = bare_vars(e) / (mode == 0 ? 1 : mode == 2 ? 4 : 2);
-    if (e->L.n_slots + bare > (mode == 0 ? kResFixedSlots : kResRuleSlots)) return false;
+    uint64_t load = e->L.n_slots + bare_vars(e) / (mode == 0 ? 1 : mode == 2 ? 4 : 2);
+    if (mode == 0 && (e->prec == 64 || e->damping != 0.0) && e->L.nf_big > e->L.nf_huge)
+        load += kResWarpSlot * (e->L.fb_off[e->L.nf_big] - e->L.fb_off[e->L.nf_huge]);
+    if (load > (mode == 0 ? kResFixedSlots : kResRuleSlots)) return false;
     if (e->res_plan < 0) {
         if (e->prec == 64) plan_resident_t<double>(e);
         else plan_resident_t<float>(e);

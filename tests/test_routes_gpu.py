@@ -31,8 +31,8 @@ def _run(e, mode):
     return info, [e.beliefs(), *([e.lowpass()] if mode == "lowpass" else []), *e.vf_messages()]
 
 
-def _check(a, prec, mode, one_launch):
-    e = Engine(a, precision=prec)
+def _check(a, prec, mode, one_launch, damping=0.0):
+    e = Engine(a, precision=prec, damping=damping)
     info, got = _run(e, mode)
     e.set_kernel_timing(True)
     _, want = _run(e, mode)
@@ -53,3 +53,13 @@ def test_variables_without_entries(prec, mode, bare, one_launch):
     a = _bingo(2500)
     a["n_vars"] += bare
     _check(a, prec, mode, one_launch)
+
+
+# graphs of 708 k and 590 k slots, 12 % of them in factors that take a warp each
+@pytest.mark.parametrize("tuples,prec,damping,mode,one_launch", [
+    (120_000, 32, 0.0, "fixed", False), (100_000, 32, 0.0, "fixed", True), (100_000, 32, 0.1, "fixed", False),
+    (100_000, 64, 0.0, "fixed", False), (100_000, 64, 0.1, "tol", True), (50_000, 64, 0.1, "fixed", True),
+])
+def test_factors_that_take_a_warp(tuples, prec, damping, mode, one_launch):
+    a = CausalFactorGraph.from_factors(workloads.config1(1, scale=tuples / 1_000_000)).graph_arrays()
+    _check(a, prec, mode, one_launch, damping)
