@@ -15,6 +15,7 @@
 #include <cstring>
 #include <limits>
 #include <atomic>
+#include <functional>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -1029,9 +1030,30 @@ int plan_cluster_t(flbp_engine *e) {
         return (uint64_t)(L.fg_base[J.fg1] - L.fg_base[J.fg0]) +
                (J.fb1 > J.fb0 ? (uint64_t)(L.fb_off[J.fb1] - L.fb_off[J.fb0]) : 0u) + bare_vars(L, J.vg0, J.vg1) / 2;
     };
+    std::vector<double> slots(all.size());
+    for (size_t k = 0; k < all.size(); k++) slots[k] = (double)job_slots(all[k]);
     std::vector<ClusterLoad> load(all.size());
     for (size_t k = 0; k < all.size(); k++)
         if (!huge[k]) load[k] = cluster_load<T>(L, all[k], damp);
+    // Sweeps of a set of graphs that run together, over those of one of them:
+    // the set goes on until its last graph has settled, and small graphs differ
+    // most (graphs of 8 k slots took 30 to 150 sweeps to 1e-6, of 42 k 30 to
+    // 65, of 400 k 32 to 40).
+    auto spread = [&](const std::vector<uint32_t> &set) {
+        double s = 1.0;
+        for (uint32_t k : set) s += std::pow(8000.0 / std::max(1.0, slots[k]), 1.5);
+        return std::min(4.0, 1.0 + 0.5 * std::log2(s));
+    };
+    // The same for graphs that run in the resident kernel or in the passes
+    // (five launches a sweep with the lists of live tiles): a part for every
+    // sweep of the set, and one for every slot while its graph is live.
+    const bool resident = e->n_graphs && use_resident(e, 3);
+    auto others = [&](const std::vector<uint32_t> &set) {
+        double n = 0.0;
+        for (uint32_t k : set) n += slots[k];
+        if (sizeof(T) == 4) return resident ? 9.4 * spread(set) + 1.3e-5 * n : 42.0 * spread(set) + 1.3e-5 * n;
+        return resident ? 9.5 * spread(set) + 2.0e-5 * n : 45.0 * spread(set) + 3.0e-5 * n;
+    };
     double best = 1e300;
     std::vector<uint32_t> best_jobs;
     for (uint32_t nb = 1; nb <= 16; nb *= 2) {
@@ -1060,20 +1082,37 @@ int plan_cluster_t(flbp_engine *e) {
         // Estimated time of a sweep of everything (us). A job's sweep is its
         // latency plus the messages a block sends, one store each at a rate
         // that measured the same from 1 k to 10 k slots a block.
-        double longest = 0.0, total = 0.0, rest = 0.0;
+        const uint32_t nclusters = (uint32_t)std::min<uint64_t>((uint64_t)nc, (uint64_t)jobs.size() * copies);
         std::vector<uint8_t> in(all.size(), 0);
+        std::vector<double> times;
         for (uint32_t k : jobs) {
-            const double n = (double)job_slots(all[k]) / nb;
-            const double t = sizeof(T) == 4 ? 5.0 + 1.75e-3 * n : 8.0 + 3.0e-3 * n;
-            longest = std::max(longest, t);
-            total += t * copies;
+            const double n = slots[k] / nb;
+            times.push_back(sizeof(T) == 4 ? 5.0 + 1.75e-3 * n : 8.0 + 3.0e-3 * n);
             in[k] = 1;
         }
-        for (uint32_t k = 0; k < all.size(); k++)
-            if (!in[k]) rest += 1.2e-5 * (double)job_slots(all[k]);
-        const uint32_t nclusters = (uint32_t)std::min<uint64_t>((uint64_t)nc, (uint64_t)jobs.size() * copies);
-        if (e->n_sets) total = longest * ((copies + nclusters - 1) / nclusters) * nclusters;  // whole rounds of like jobs
-        const double t = std::max(longest, total / nclusters) + (rest > 0.0 ? 8.0 + rest : 0.0);
+        const double longest = *std::max_element(times.begin(), times.end());
+        double t = longest;
+        if (e->n_sets) {  // whole rounds of like jobs
+            t = longest * ((copies + nclusters - 1) / nclusters);
+        } else if (e->n_graphs) {
+            // the clusters' shares when every job goes to the one that is free first, the longest
+            // first; or the graph that needs most sweeps, most likely one of the smallest
+            std::sort(times.begin(), times.end(), std::greater<double>());
+            std::priority_queue<double, std::vector<double>, std::greater<double>> ends;
+            for (double x : times) {
+                double from = 0.0;
+                if (ends.size() == nclusters) {
+                    from = ends.top();
+                    ends.pop();
+                }
+                ends.push(from + x);
+                t = std::max(t, from + x);
+            }
+            std::vector<uint32_t> rest;
+            for (uint32_t k = 0; k < all.size(); k++)
+                if (!in[k]) rest.push_back(k);
+            t = std::max(t, times.back() * spread(jobs)) + (rest.empty() ? 0.0 : others(rest));
+        }
         if (t >= best) continue;
         best = t;
         best_jobs = jobs;
@@ -1084,6 +1123,17 @@ int plan_cluster_t(flbp_engine *e) {
         e->cl_smem = smem;
     }
     if (best_jobs.empty()) return FLBP_OK;
+    // Batches go to clusters where that is estimated faster than all of their
+    // graphs in the other form. Measured, ms of a batch to 1e-6 on clusters and
+    // in that form: 48 graphs of 8 k slots 1.5 : 1.9 (resident), of 21 k 1.2 :
+    // 4.8 (passes), 8 of 42 k 0.68 : 0.57, 4 of 134 k 0.76 : 0.63; FP64 8 of
+    // 21 k 0.83 : 0.68, 1 of 100 k 1.04 : 0.45, 16 of 67 k 1.9 : 2.8 (passes);
+    // 5,600 of 0.5 k 6.7 : 4.6 (passes).
+    if (e->n_graphs) {
+        std::vector<uint32_t> every(all.size());
+        std::iota(every.begin(), every.end(), 0u);
+        if (best >= others(every)) return FLBP_OK;
+    }
     // Few large evidence sets leave clusters idle; the direct form takes
     // about 20 us and 16.5 us per million slots (48 sets of 158 k slots: 4.9 ms
     // in either form, 8 of them 1.13 ms direct and 1.30 ms on clusters).

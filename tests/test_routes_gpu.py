@@ -6,7 +6,7 @@ the same results either way (per-pass timing mode forces the passes).
 import numpy as np
 import pytest
 
-from fastlbp_b200 import CausalFactorGraph, Engine, workloads
+from fastlbp_b200 import BatchEngine, CausalFactorGraph, Engine, workloads
 
 pytestmark = pytest.mark.gpu
 
@@ -63,3 +63,46 @@ def test_variables_without_entries(prec, mode, bare, one_launch):
 def test_factors_that_take_a_warp(tuples, prec, damping, mode, one_launch):
     a = CausalFactorGraph.from_factors(workloads.config1(1, scale=tuples / 1_000_000)).graph_arrays()
     _check(a, prec, mode, one_launch, damping)
+
+
+def _batch(graphs, prec, sweeps, passes=False):
+    e = BatchEngine(graphs, precision=prec)
+    e.set_kernel_timing(passes)
+    e.init()
+    stops = e.run_batch_tol(1e-6, sweeps)
+    info = e.info.as_dict()
+    out = [e.beliefs(), *stops, [info[k] for k in ("sweeps", "reason", "maxdiff")], *e.vf_messages()]
+    e.close()
+    return info, out
+
+
+# batches on clusters or resident, on clusters with the rest in the passes, and all in the passes
+@pytest.mark.parametrize("prec", [32, 64])
+@pytest.mark.parametrize("sizes,one_launch", [
+    ([300] * 5 + [1000] * 3, True), ([9000, 9100, 9200], True),
+    ([1000 + k for k in range(24)] + [70_000, 71_000], False), ([60_000, 61_000, 62_000], False),
+], ids=["small", "resident", "both", "passes"])
+def test_batches(prec, sizes, one_launch):
+    graphs = [_bingo(n, seed=k + 1) for k, n in enumerate(sizes)]
+    info, got = _batch(graphs, prec, 25)
+    _, want = _batch(graphs, prec, 25, passes=True)
+    assert all(np.array_equal(x, y, equal_nan=True) for x, y in zip(got, want))
+    assert (info["launches"] == 1) == one_launch
+
+
+def test_thousands_of_tiny_graphs():
+    """More graphs than clusters take in a reasonable number of rounds, and than the resident kernel counts."""
+    kinds = [_bingo(60 + k, seed=k + 1) for k in range(7)]
+    info, got = _batch(kinds * 800, 32, 40)
+    assert info["launches"] > 1
+    n = sum(a["n_vars"] for a in kinds)
+    alone, sweeps = [], []
+    for a in kinds:
+        e = Engine(a)
+        e.init()
+        sweeps.append(e.run_tol(1e-6, 40, 1e9)["sweeps"])
+        alone.append(e.beliefs())
+        e.close()
+    for at in (0, 399, 799):
+        assert np.array_equal(got[0][at * n:(at + 1) * n], np.concatenate(alone))
+    assert list(got[1]) == sweeps * 800
