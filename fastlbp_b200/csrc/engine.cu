@@ -1135,9 +1135,10 @@ int plan_cluster_t(flbp_engine *e) {
         if (best >= others(every)) return FLBP_OK;
     }
     // Few large evidence sets leave clusters idle; the direct form takes
-    // about 20 us and 16.5 us per million slots (48 sets of 158 k slots: 4.9 ms
-    // in either form, 8 of them 1.13 ms direct and 1.30 ms on clusters).
-    if (e->n_sets && best > 20.0 + 1.65e-5 * (double)L.n_slots * e->n_sets) return FLBP_OK;
+    // about 19 us and 16.5 us per million slots (48 sets of 158 k slots: 4.9 ms
+    // in either form, 8 of them 1.13 ms direct and 1.30 ms on clusters, one
+    // 0.68 and 0.73, two 0.80 and 0.74).
+    if (e->n_sets && best > 19.0 + 1.65e-5 * (double)L.n_slots * e->n_sets) return FLBP_OK;
     // largest first
     std::stable_sort(best_jobs.begin(), best_jobs.end(),
                      [&](uint32_t x, uint32_t y) { return items_v(all[x]) > items_v(all[y]); });

@@ -6,7 +6,7 @@ the same results either way (per-pass timing mode forces the passes).
 import numpy as np
 import pytest
 
-from fastlbp_b200 import BatchEngine, CausalFactorGraph, Engine, workloads
+from fastlbp_b200 import BatchEngine, CausalFactorGraph, Engine, SetsEngine, workloads
 
 pytestmark = pytest.mark.gpu
 
@@ -106,3 +106,19 @@ def test_thousands_of_tiny_graphs():
     for at in (0, 399, 799):
         assert np.array_equal(got[0][at * n:(at + 1) * n], np.concatenate(alone))
     assert list(got[1]) == sweeps * 800
+
+
+@pytest.mark.parametrize("tuples,n_sets,one_launch", [(2000, 1, True), (20_000, 1, False), (20_000, 3, True)])
+def test_evidence_sets(tuples, n_sets, one_launch):
+    sets = [{3: 1, 10 + k: k % 2} for k in range(n_sets)]
+    got = []
+    for passes in (False, True):
+        e = SetsEngine(_bingo(tuples), sets)
+        e.set_kernel_timing(passes)
+        e.init()
+        stops = e.run_sets_tol(1e-6, 25)
+        got.append([e.beliefs(), *stops])
+        if not passes:
+            assert (e.info.as_dict()["launches"] == 1) == one_launch
+        e.close()
+    assert all(np.array_equal(x, y, equal_nan=True) for x, y in zip(*got))
