@@ -997,6 +997,12 @@ size_t cluster_job_smem(const HostLayout &L, const ClusterJob &J, const ClusterL
     return bytes <= kClusterSmemMax ? bytes : 0;
 }
 
+// Bit e of set k's `words` words: no message reaches entry e. cut: (set, entry) pairs.
+__global__ void cut_bits_kernel(const uint2 *__restrict__ cut, uint32_t n, uint32_t words, uint32_t *__restrict__ bits) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) atomicOr(bits + (size_t)cut[i].x * words + (cut[i].y >> 5), 1u << (cut[i].y & 31u));
+}
+
 // Cluster size and jobs of this engine, or a plan of 0.
 template <typename T>
 int plan_cluster_t(flbp_engine *e) {
@@ -1160,17 +1166,30 @@ int plan_cluster_t(flbp_engine *e) {
     e->cl_all = jobs.size() == all.size() * copies;
     const size_t groups = std::max<size_t>({1, e->n_sets, e->n_graphs});
     const size_t bytes = e->bytes;
+    // the cut entries of every set as bits: only for engines that run on clusters, since it is a bit for
+    // every entry of every set
+    e->cut_words = e->n_set_cut ? (uint32_t)((e->n_ent + 31) / 32) : 0u;
+    const size_t cut_bits = (size_t)e->n_sets * e->cut_words;
     if (dalloc(e, &e->d_cl_jobs, jobs.size()) || dalloc(e, &e->d_cl_map, (size_t)e->cl_map_words * e->cl_clusters) ||
-        dalloc(e, &e->d_gdiff, groups)) {  // no memory for this kernel's tables: the passes need none
+        dalloc(e, &e->d_gdiff, groups) || (cut_bits && dalloc(e, &e->d_cut_ent, cut_bits))) {
+        // no memory for this kernel's tables: the passes need none
         cudaGetLastError();
         dfree(e, e->d_cl_jobs);
         dfree(e, e->d_cl_map);
         dfree(e, e->d_gdiff);
+        dfree(e, e->d_cut_ent);
         e->d_cl_jobs = nullptr;
         e->d_cl_map = nullptr;
         e->d_gdiff = nullptr;
+        e->d_cut_ent = nullptr;
         e->bytes = bytes;
         return FLBP_OK;
+    }
+    if (cut_bits) {
+        FLBP_CUDA(cudaMemsetAsync(e->d_cut_ent, 0, cut_bits * sizeof(uint32_t), e->stream));
+        cut_bits_kernel<<<(e->n_set_cut + 255) / 256, 256, 0, e->stream>>>(e->d_set_cut, e->n_set_cut, e->cut_words,
+                                                                          e->d_cut_ent);
+        FLBP_CUDA(cudaGetLastError());
     }
     if (int rc = upload(e, e->d_cl_jobs, jobs)) return rc;
     FLBP_CUDA(cudaStreamSynchronize(e->stream));  // the job list is a local of this function
@@ -3942,12 +3961,6 @@ int flbp_sets_create(const flbp_graph_desc *graph, int64_t n_sets, const int64_t
         (!cut.empty() && ((rc = dalloc(e, &e->d_set_cut, cut.size())) || (rc = upload(e, e->d_set_cut, cut)))) ||
         (!slots.empty() && ((rc = dalloc(e, &e->d_set_slots, slots.size())) || (rc = upload(e, e->d_set_slots, slots)))))
         return fail(rc);
-    if (!cut.empty()) {  // the cut entries as bits, for the cluster kernel
-        e->cut_words = (uint32_t)((ne + 31) / 32);
-        std::vector<uint32_t> bits((size_t)S * e->cut_words, 0u);
-        for (const uint2 &c : cut) bits[(size_t)c.x * e->cut_words + (c.y >> 5)] |= 1u << (c.y & 31u);
-        if ((rc = dalloc(e, &e->d_cut_ent, bits.size())) || (rc = upload(e, e->d_cut_ent, bits))) return fail(rc);
-    }
     FLBP_CUDA(cudaMemsetAsync(e->d_belief, 0, S * nv_pad * sizeof(double), e->stream));
     FLBP_CUDA(cudaMemsetAsync(e->d_gstate, 0, 4 * sizeof(int) * S, e->stream));
     FLBP_CUDA(cudaStreamSynchronize(e->stream));
