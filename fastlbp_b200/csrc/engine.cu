@@ -1945,41 +1945,36 @@ int create_engine(const flbp_graph_desc *graph, const flbp_engine_opts *opts, fl
         e->n_graphs = (uint32_t)(batch->var_off.size() - 1);
         e->graph_var_off = batch->var_off;
         std::vector<uint32_t> fg(nf_pad, 0), vg(std::max<size_t>(1, nv_pad), 0);
-        for (uint32_t f = 0; f < nf; f++) fg[f] = batch->factor_graph[L.factor_of_internal[f]];
-        for (uint32_t iv = 0; iv < (uint32_t)L.V; iv++) vg[iv] = batch->var_graph[L.var_of_internal[iv]];
-        {  // every graph's items, for the cluster kernel
+        {  // with every graph's items, for the cluster kernel: the layout keeps those of a class together
             const uint32_t ng = e->n_graphs;
             std::vector<ClusterJob> &J = e->batch_jobs;
             J.assign(ng, ClusterJob{});
             e->batch_huge.assign(ng, 0);
-            for (uint32_t f = 0; f < L.nf_sell; f++) {
-                ClusterJob &j = J[fg[f]];
-                if (j.f_hi == 0) j.f_lo = f;
-                j.f_hi = f + 1;
-            }
-            for (uint32_t v = 0; v < L.nv_sell; v++) {
-                ClusterJob &j = J[vg[v]];
-                if (j.v_hi == 0) j.v_lo = v;
-                j.v_hi = v + 1;
-            }
-            for (uint32_t b = 0; b < L.nf_big; b++) {
-                const uint32_t g = fg[L.nf_sell + b];
-                if (b < L.nf_huge) {
-                    e->batch_huge[g] = 1;
-                } else {
-                    if (J[g].fb1 == 0) J[g].fb0 = b;
-                    J[g].fb1 = b + 1;
+            typedef uint32_t ClusterJob::*Bound;
+            auto fill = [&](std::vector<uint32_t> &ids, uint32_t from, uint32_t to, uint32_t base, Bound lo, Bound hi,
+                            auto graph_of) {
+                uint32_t prev = ng;
+                for (uint32_t i = from; i < to; i++) {
+                    const uint32_t g = ids[i] = graph_of(i);
+                    if (g == prev) continue;
+                    if (prev < ng) J[prev].*hi = i - base;
+                    J[g].*lo = i - base;
+                    prev = g;
                 }
-            }
-            for (uint32_t b = 0; b < L.nv_big; b++) {
-                const uint32_t g = vg[L.nv_sell + b];
-                if (b < L.nv_huge) {
-                    e->batch_huge[g] = 1;
-                } else {
-                    if (J[g].vb1 == 0) J[g].vb0 = b;
-                    J[g].vb1 = b + 1;
-                }
-            }
+                if (prev < ng) J[prev].*hi = to - base;
+            };
+            auto fill_huge = [&](std::vector<uint32_t> &ids, uint32_t from, uint32_t to, auto graph_of) {
+                for (uint32_t i = from; i < to; i++) e->batch_huge[ids[i] = graph_of(i)] = 1;
+            };
+            auto f_of = [&](uint32_t f) { return batch->factor_graph[L.factor_of_internal[f]]; };
+            auto v_of = [&](uint32_t v) { return batch->var_graph[L.var_of_internal[v]]; };
+            const uint32_t fs = L.nf_sell, fh = fs + L.nf_huge, vs = L.nv_sell, vh = vs + L.nv_huge;
+            fill(fg, 0, fs, 0, &ClusterJob::f_lo, &ClusterJob::f_hi, f_of);
+            fill_huge(fg, fs, fh, f_of);
+            fill(fg, fh, fs + L.nf_big, fs, &ClusterJob::fb0, &ClusterJob::fb1, f_of);
+            fill(vg, 0, vs, 0, &ClusterJob::v_lo, &ClusterJob::v_hi, v_of);
+            fill_huge(vg, vs, vh, v_of);
+            fill(vg, vh, vs + L.nv_big, vs, &ClusterJob::vb0, &ClusterJob::vb1, v_of);
             for (uint32_t g = 0; g < ng; g++) {
                 J[g].fg0 = J[g].f_lo / 32;
                 J[g].fg1 = (J[g].f_hi + 31) / 32;
