@@ -116,6 +116,8 @@ struct flbp_engine {
     double *d_adj_in = nullptr, *d_adj_out = nullptr;         // staging of the host-buffer backward call
     uint32_t *d_adj_groups = nullptr;  // sliced-ELL group ids by width class (see adj_group_n)
     double *d_ref_out = nullptr;       // per-variable results in the caller's order (readback staging)
+    double *d_sets_out = nullptr;      // the same for several evidence sets at once (null: one at a time)
+    int64_t sets_out_n = 0;            // values it holds
     uint32_t adj_group_n[4] = {0, 0, 0, 0};
     std::vector<double> factor_p_host;  // every reference factor's p (for derivatives of folded constants)
     std::vector<double> factor_q_host;  // every reference factor's q
@@ -2155,7 +2157,7 @@ int flbp_engine_destroy(flbp_engine *e) {
                     e->d_fbt_kind, e->d_fbt_pq, e->d_vbt_prior, e->d_f_graph, e->d_v_graph, e->d_gstate, e->d_ftrange, e->d_vtrange,
                     e->d_ckpt, e->d_seg_vf, e->d_seg_fv, e->d_lam, e->d_lam2, e->d_mu, e->d_gp, e->d_gq,
                     e->d_gprior, e->d_gs, e->d_int_of_var, e->d_f_of_int, e->d_pri_fac, e->d_pri_var, e->d_pri_coef,
-                    e->d_adj_in, e->d_adj_out, e->d_adj_groups, e->d_ref_out, e->d_clamp_slots, e->d_clamp_upd,
+                    e->d_adj_in, e->d_adj_out, e->d_adj_groups, e->d_ref_out, e->d_sets_out, e->d_clamp_slots, e->d_clamp_upd,
                     e->d_sq_foff, e->d_sq_var, e->d_sq_items, e->d_sq_tgt, e->d_sq_iota, e->d_sq_kind,
                     e->d_sq_cst, e->d_sq_pq, e->d_sq_fv, e->d_sq_vf, e->d_sq_nw, e->d_sq_S, e->d_sq_cnt};
     for (void *b : bufs)
@@ -2387,18 +2389,33 @@ static int fetch_internal(flbp_engine *e, const double *dsrc, double *out, int64
         std::vector<uint32_t> iov(e->L.internal_of_var.begin(), e->L.internal_of_var.end());
         if ((rc = dalloc(e, &e->d_int_of_var, iov.size())) || (rc = upload(e, e->d_int_of_var, iov))) return rc;
     }
-    const int64_t per = std::min(sets, std::max<int64_t>(1, kFetchValues / n));
-    if (!e->d_ref_out && (rc = dalloc(e, &e->d_ref_out, (size_t)(per * n)))) return rc;
+    if (!e->d_ref_out && (rc = dalloc(e, &e->d_ref_out, (size_t)n))) return rc;
+    int64_t per = std::min(sets, std::max<int64_t>(1, kFetchValues / n));
+    double *buf = e->d_ref_out;
+    if (per > 1) {  // without memory for several sets one after the other, which needs no more
+        if (!e->d_sets_out) {
+            const size_t bytes = e->bytes;
+            if (dalloc(e, &e->d_sets_out, (size_t)(per * n))) {
+                cudaGetLastError();
+                e->d_sets_out = nullptr;
+                e->bytes = bytes;
+            } else {
+                e->sets_out_n = per * n;
+            }
+        }
+        per = std::max<int64_t>(1, std::min(per, e->sets_out_n / n));
+        if (per > 1) buf = e->d_sets_out;
+    }
     PinnedStage *S = per * n >= (1 << 16) ? stage_for(e->device) : nullptr;  // large outputs through the staging buffers
     std::unique_lock<std::mutex> lock;
     if (S) lock = std::unique_lock<std::mutex>(S->mu);
     for (int64_t k = 0; k < sets; k += per) {
         const int64_t m = std::min(per, sets - k);
         gather_vars_kernel<<<dim3((unsigned)((n + 255) / 256), (unsigned)m), 256, 0, e->stream>>>(
-            dsrc + (uint64_t)k * stride, stride, e->d_int_of_var, n, e->d_ref_out);
+            dsrc + (uint64_t)k * stride, stride, e->d_int_of_var, n, buf);
         e->launches += 1;
         FLBP_CUDA(cudaGetLastError());
-        FLBP_CUDA(staged_d2h<double>(e, S, out + k * n, e->d_ref_out, (size_t)(m * n)));
+        FLBP_CUDA(staged_d2h<double>(e, S, out + k * n, buf, (size_t)(m * n)));
     }
     return FLBP_OK;
 }
@@ -3943,7 +3960,7 @@ int flbp_sets_create(const flbp_graph_desc *graph, int64_t n_sets, const int64_t
     }
     // S copies of the run state; the layout stays single
     for (void **b : {(void **)&e->d_vf, (void **)&e->d_fv, (void **)&e->d_fvd, (void **)&e->d_belief,
-                     (void **)&e->d_prior, (void **)&e->d_gstate, (void **)&e->d_ref_out})
+                     (void **)&e->d_prior, (void **)&e->d_gstate})
         if (*b) {
             dfree(e, *b);
             *b = nullptr;
