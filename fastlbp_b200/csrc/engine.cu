@@ -2159,7 +2159,8 @@ int flbp_engine_destroy(flbp_engine *e) {
                     e->d_gprior, e->d_gs, e->d_int_of_var, e->d_f_of_int, e->d_pri_fac, e->d_pri_var, e->d_pri_coef,
                     e->d_adj_in, e->d_adj_out, e->d_adj_groups, e->d_ref_out, e->d_sets_out, e->d_clamp_slots, e->d_clamp_upd,
                     e->d_sq_foff, e->d_sq_var, e->d_sq_items, e->d_sq_tgt, e->d_sq_iota, e->d_sq_kind,
-                    e->d_sq_cst, e->d_sq_pq, e->d_sq_fv, e->d_sq_vf, e->d_sq_nw, e->d_sq_S, e->d_sq_cnt};
+                    e->d_sq_cst, e->d_sq_pq, e->d_sq_fv, e->d_sq_vf, e->d_sq_nw, e->d_sq_S, e->d_sq_cnt,
+                    e->d_sq_irec, e->d_sq_tvar, e->d_sq_tst, e->d_sq_bo};
     for (void *b : bufs)
         if (b) cudaFree(b);
     for (void *b : e->d_in)
