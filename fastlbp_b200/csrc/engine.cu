@@ -3121,11 +3121,6 @@ char *adj_seg_fv(flbp_engine *e, long long i) {
     return (char *)e->d_seg_fv + (size_t)i * std::max<size_t>(1, e->n_ent) * e->tsize;
 }
 
-// The checkpointed forward run on explicit buffers: each segment's sweeps
-// start from its checkpoint, the last sweep of a segment writes the next
-// checkpoint, and the last segment keeps every state in the segment buffers
-// (its final variable pass writes the engine's vf, and fv_{T-1} is copied
-// to the engine's fv, so the engine state is that of T plain sweeps).
 // n sweeps of a segment from v0: f->v messages of sweep i to fseg + i
 // fstride, v->f messages to vseg + (i + 1) vstride (elements), the last ones
 // to vlast (null: none). One launch of the resident kernel where the graph
@@ -3164,6 +3159,11 @@ int adjoint_sweeps(flbp_engine *e, long long n, const T *v0, T *vseg, size_t vst
     return FLBP_OK;
 }
 
+// The checkpointed forward run on explicit buffers: each segment's sweeps
+// start from its checkpoint, the last sweep of a segment writes the next
+// checkpoint, and the last segment keeps every state in the segment buffers
+// (its final variable pass writes the engine's vf, and fv_{T-1} is copied
+// to the engine's fv, so the engine state is that of T plain sweeps).
 template <typename T>
 int adjoint_forward_t(flbp_engine *e, long long T_, long long K) {
     const size_t ns = std::max<uint64_t>(1, e->L.n_slots);

@@ -31,9 +31,6 @@
 
 namespace flbp {
 
-// Control block of one engine (device memory). Written by block 0 of the
-// factor pass (sweep counters, residual reset) and by the last block of the
-// variable pass (stop decision); read by every block at kernel entry.
 constexpr int kGroupWords = 128;  // groups that stop by themselves in one resident kernel, / 32
 
 // Grid-wide state of the resident run kernel (resident.cuh), zero before
@@ -56,6 +53,10 @@ struct ResSync {
 constexpr unsigned int kResMoved = 1u << 12, kResTimeUp = 1u << 24;
 constexpr unsigned int kResMaxBlocks = kResMoved - 1u;  // both counts of an end word have 12 bits
 
+// Control block of one engine (device memory). Written by block 0 of the
+// factor pass (sweep counters, residual reset) and by the last block of the
+// variable pass (stop decision); read by every block at kernel entry. The
+// whole-run kernels (resident.cuh, resident_cluster.cuh) write it as they end.
 struct Ctl {
     unsigned long long maxdiff_bits;  // max |belief change| of this sweep, double bits
     unsigned long long nonconv;       // variables with |belief change| > tol
@@ -910,12 +911,12 @@ __device__ __forceinline__ void factor_tile_big(VB vb, const uint32_t *ps, uint3
     }
 }
 
+constexpr uint32_t kHugeRegs = 4;  // slots of a thread of factor_block_huge whose loads are in flight together
+
 // A factor too large for a tile (big factor b, internal index nf_sell + b),
 // spread over all consumer threads of a block (called by all of them): a
 // log-sigmoid sum of the body (WideAcc) with a count of -inf terms, reduced
 // over the block in a fixed order, then every slot removes its own term.
-constexpr uint32_t kHugeRegs = 4;
-
 template <typename T, typename VB>
 __device__ void factor_block_huge(const FactorArgs &a, uint32_t b, int tid, VB vf, T *__restrict__ fv,
                                   typename WideAcc<T>::type *s_l, int *s_nz) {
@@ -1217,12 +1218,6 @@ __device__ __forceinline__ T take_fv(T x, T old, T d) {
 template <typename T, bool DAMP>
 __device__ __forceinline__ T take_fv_fin(T x, T old, T d) {
     return DAMP ? fma(T(1) - d, x, d * old) : x;
-}
-
-// Finite (neither +-inf nor NaN).
-template <typename T>
-__device__ __forceinline__ bool is_fin(T x) {
-    return fabs(x) < Num<T>::inf();
 }
 
 // Sum of one sliced-ELL variable (one lane) whose new messages are x[0..w)

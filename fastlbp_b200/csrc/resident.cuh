@@ -38,7 +38,7 @@
 namespace flbp {
 
 constexpr int kResThreads = kConsumers;   // 16 warps: the huge-item paths synchronise all consumer threads
-constexpr uint32_t kResMaxRows = 512;     // items of a pass per block with cached constants
+constexpr uint32_t kResMaxRows = 512;     // items of both passes together per block with cached constants
 
 template <typename T>
 struct ResArgs {
