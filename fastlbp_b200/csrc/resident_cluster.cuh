@@ -23,10 +23,11 @@
 // (about 0.8 us with its fences) on the smallest graphs, on larger ones the
 // remote stores, which an SM sends and takes in at about one in two cycles -
 // no faster than L2 takes scattered stores, so that a graph spread over 16
-// blocks gains nothing above some 40 k slots. Measured (FP32, one B200): 30
-// tolerance sweeps of 16 k slots 288 -> 206 us; 64 evidence sets of 12 k
-// slots 2.34 -> 0.99 ms; 64 graphs of 500 to 1,000 tuples 5.4 -> 3.0 ms; 48
-// graphs of 1 k to 50 k tuples, of which 36 fit, 8.5 -> 5.1 ms.
+// blocks gains nothing above some 40 k slots. Measured on one B200 in FP32,
+// whole calls, the two launches a sweep against this kernel: 30 tolerance
+// sweeps of 17 k slots 0.51 : 0.25 ms; 64 evidence sets of 12 k slots 2.2 :
+// 0.86 ms; 64 graphs of 500 to 1,000 tuples 3.7 : 0.71 ms; 48 graphs of 1 k to
+// 50 k tuples, the larger ones in the passes, 8.8 : 6.6 ms.
 //
 // Items are evaluated by the functions of the pass kernels in the same order
 // per item, so a run gives the same bits as the other forms. Messages,
