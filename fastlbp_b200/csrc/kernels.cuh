@@ -1585,9 +1585,12 @@ __device__ __forceinline__ void var_close(const VarArgs &a, Ctl *ctl, double dma
 // tile are taken first, one per warp. With BMODE 1/2 the
 // block maxima of |belief change| are combined with an atomic max and the
 // last block to finish applies the stop rules. DAMP mixes each new message
-// with the previous damped one (fvd) and stores the result back to fvd.
+// with the previous damped one (fvd) and stores the result back to fvd. Two
+// blocks per SM are what the stages leave room for; said so, the compiler keeps
+// 54 to 56 registers in every instance (left to itself it took 32, with spills,
+// for damped FP64: 40 sweeps of 1.7 M slots 2.89 ms against 2.77).
 template <typename T, int BMODE, bool WRITE_VF, bool DAMP, int STAGES>
-__global__ void __launch_bounds__(kBlockThreadsDev) var_pass_kernel(VarArgs a, const T *__restrict__ fv,
+__global__ void __launch_bounds__(kBlockThreadsDev, 2) var_pass_kernel(VarArgs a, const T *__restrict__ fv,
                                                                     T *__restrict__ vf, T *__restrict__ fvd, T d,
                                                                     Ctl *ctl) {
     extern __shared__ __align__(128) unsigned char smem[];
